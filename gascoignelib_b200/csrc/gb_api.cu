@@ -32,7 +32,7 @@ gb_ctx_create(gb_ctx** out, int device)
     if (const char* e = getenv("GB_ROW_ORDER"))
       ctx->row_order = atoi(e) != 0;
     if (const char* e = getenv("GB_ILU_CTA_ROWS"))
-      ctx->ilu_cta_rows = std::max(0, atoi(e));
+      ctx->ilu_cta_rows = std::max(0, atoi(e)), ctx->ilu_cluster = false;
     if (const char* e = getenv("GB_VANKA_HOST"))
       ctx->vanka_host = atoi(e) != 0;
     if (const char* e = getenv("GB_CLUSTER"))
@@ -104,6 +104,7 @@ gb_ctx_synchronize(gb_ctx* ctx)
 {
   GB_API_BEGIN
   GB_CUDA(cudaStreamSynchronize(ctx->stream));
+  throw_if_wait_ended(*ctx);
   GB_API_END
 }
 
@@ -421,6 +422,7 @@ gb_vec_download(gb_ctx* ctx, int lvl, int id, double* host, int64_t len)
   GB_CUDA(cudaMemcpyAsync(host, d, len * sizeof(double), cudaMemcpyDeviceToHost,
                           ctx->stream));
   GB_CUDA(cudaStreamSynchronize(ctx->stream));
+  throw_if_wait_ended(*ctx);
   GB_API_END
 }
 

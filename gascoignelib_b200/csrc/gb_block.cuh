@@ -3,6 +3,7 @@
 // Included by gb_context.cuh after gb_kernels.cuh.
 #pragma once
 #include "gb_kernels.cuh"
+#include <type_traits>
 
 namespace gb {
 
@@ -778,7 +779,8 @@ k_to_float(int64_t n, const double* __restrict__ a, float* __restrict__ b)
 // subtractions run in the reference's order, so a row waits for about two
 // memory round trips per G entries instead of one per entry. The rows of one
 // dependency level depend only on rows of earlier levels, so running the
-// levels in order gives the sequential sweep bit for bit.
+// levels in order gives the sequential sweep bit for bit. (Levels too large for
+// k_ilu_cluster.)
 template<int B, class T, bool UP>
 __device__ __forceinline__ void
 ilu_row(int i, const int* __restrict__ ptr, const int* __restrict__ col,
@@ -899,6 +901,353 @@ k_ilu_levels(int lv0, int lv1, const int* __restrict__ lptr, const int* __restri
     o0 = o1;
     o1 = o2;
   }
+}
+
+// ------------------------------------- both substitutions in one cluster
+//
+// A packed copy of the factors for k_ilu_cluster, one per direction (0 forward,
+// 1 backward). CTA r of the cluster owns the rows [r chunk, (r + 1) chunk). Its
+// rows are put in groups of 32 (one per lane) of one dependency level each, the
+// groups in level order: group g's lane l works on row[32 g + l] (-1: none).
+// base[g] >> 1 is the group's first entry, bit 0 whether some entry is in
+// another CTA's rows. A row's entries are in the substitution's order at the
+// end of the group's width, a multiple of ilu_half(B); before them it has entries
+// of value 0 and a column that is always there (place chunk * B of the own
+// CTA, which holds zeros). A column is coded owner << 24 | place of its first
+// component; its block follows component-major.
+template<class T>
+struct IluPack
+{
+  int chunk;
+  const int *gptr, *row, *base, *col;
+  const T* val;
+  const T* dinv; // backward only: the inverted diagonal blocks
+};
+
+constexpr int kIluOwnerShift = 24;
+constexpr int kIluPlaceMask = (1 << kIluOwnerShift) - 1;
+
+// The "not yet computed" mark of a word of y: all bits set, a NaN. It is told
+// by the upper 32 bits, and a computed value with such bits is stored as
+// another NaN.
+template<class T>
+struct IluWord;
+template<>
+struct IluWord<float>
+{
+  using U = uint32_t;
+  static constexpr U kMark = 0xffffffffu, kNaN = 0x7fffffffu;
+  static __device__ __forceinline__ U bits(float v) { return __float_as_uint(v); }
+  static __device__ __forceinline__ float value(U u) { return __uint_as_float(u); }
+  static __device__ __forceinline__ uint32_t upper(U u) { return u; }
+  template<bool FAR>
+  static __device__ __forceinline__ U load(uint32_t a)
+  {
+    U v;
+    if (FAR)
+      asm volatile("ld.relaxed.cluster.shared::cluster.u32 %0, [%1];" : "=r"(v) : "r"(a) : "memory");
+    else
+      asm volatile("ld.relaxed.cluster.shared::cta.u32 %0, [%1];" : "=r"(v) : "r"(a) : "memory");
+    return v;
+  }
+  static __device__ __forceinline__ void store(uint32_t a, U v)
+  {
+    asm volatile("st.relaxed.cluster.shared::cta.u32 [%0], %1;" ::"r"(a), "r"(v) : "memory");
+  }
+};
+template<>
+struct IluWord<double>
+{
+  using U = unsigned long long;
+  static constexpr U kMark = 0xffffffffffffffffull, kNaN = 0x7fffffffffffffffull;
+  static __device__ __forceinline__ U bits(double v) { return __double_as_longlong(v); }
+  static __device__ __forceinline__ double value(U u) { return __longlong_as_double(u); }
+  static __device__ __forceinline__ uint32_t upper(U u) { return uint32_t(u >> 32); }
+  template<bool FAR>
+  static __device__ __forceinline__ U load(uint32_t a)
+  {
+    U v;
+    if (FAR)
+      asm volatile("ld.relaxed.cluster.shared::cluster.u64 %0, [%1];" : "=l"(v) : "r"(a) : "memory");
+    else
+      asm volatile("ld.relaxed.cluster.shared::cta.u64 %0, [%1];" : "=l"(v) : "r"(a) : "memory");
+    return v;
+  }
+  static __device__ __forceinline__ void store(uint32_t a, U v)
+  {
+    asm volatile("st.relaxed.cluster.shared::cta.u64 [%0], %1;" ::"r"(a), "l"(v) : "memory");
+  }
+};
+
+// entries consumed together: their blocks and y in registers
+__host__ __device__ constexpr int
+ilu_half(int B)
+{
+  return B == 1 ? 8 : B == 2 ? 4 : 2;
+}
+
+// The packed layout from the row-sorted factors, one warp per group; col is
+// null when only the values changed.
+template<class T, bool UP>
+__global__ void
+k_ilu_pack(int ngroups, int B, int chunk, const int* __restrict__ row,
+           const int* __restrict__ base, const int* __restrict__ ptr,
+           const int* __restrict__ fcol, const int* __restrict__ diag,
+           const double* __restrict__ v, const int* __restrict__ gptr,
+           int* __restrict__ col, T* __restrict__ val, T* __restrict__ dinv)
+{
+  GB_PDL_ENTRY();
+  const int lane = threadIdx.x & 31, B2 = B * B;
+  const int g = static_cast<int>((blockIdx.x * int64_t(blockDim.x) + threadIdx.x) >> 5);
+  if (g >= ngroups)
+    return;
+  int rank = 0;
+  while (g >= gptr[rank + 1])
+    ++rank;
+  const int i = row[int64_t(g) * kSlice + lane];
+  const int e0 = base[g] >> 1, w = (base[g + 1] >> 1) - e0;
+  const int d = i < 0 ? 0 : diag[i];
+  const int first = i < 0 ? 0 : (UP ? ptr[i + 1] - 1 : ptr[i]);
+  const int cnt = i < 0 ? 0 : (UP ? first - d : d - first);
+  const int pad = w - cnt;
+  for (int e = 0; e < w; ++e) {
+    const int64_t at = int64_t(e0) + e;
+    const int p = UP ? first - (e - pad) : first + (e - pad);
+    if (col) {
+      const int k = e < pad ? 0 : fcol[p];
+      col[at * kSlice + lane] = e < pad ? (rank << kIluOwnerShift) | (chunk * B)
+                                        : ((k / chunk) << kIluOwnerShift) | ((k % chunk) * B);
+    }
+    for (int q = 0; q < B2; ++q)
+      val[(at * B2 + q) * kSlice + lane] =
+        e < pad ? T(0) : static_cast<T>(v[int64_t(p) * B2 + q]);
+  }
+  if (UP)
+    for (int q = 0; q < B2; ++q)
+      dinv[(int64_t(g) * B2 + q) * kSlice + lane] =
+        i < 0 ? T(0) : static_cast<T>(v[int64_t(d) * B2 + q]);
+}
+
+constexpr int kIluClusterThreads = 512;
+constexpr size_t kIluClusterBytes = 216 * 1024; // of y in a CTA's shared memory
+constexpr int kIluGroupsPerLevel = 2;           // a CTA's share of an average level
+constexpr int kIluClusterMax = 16;              // CTAs (16: not a portable size)
+
+// One direction of k_ilu_cluster: this CTA's groups, warp by warp in level
+// order. in: the rows' right-hand side; out: the result in global memory. All
+// that does not depend on other rows (columns, values, addresses) is done
+// before a group waits; from the moment its last dependency is stored to its
+// own store there is one poll, one read of 8 entries and their multiply-adds.
+template<int B, class T, bool UP>
+__device__ __forceinline__ void
+ilu_cluster_run(const IluPack<T>& A, uint32_t y, int rank, const T* in, T* out, T* u, T omega,
+                bool u_zero, volatile int* give_up, unsigned long long wait_ns)
+{
+  using W = IluWord<T>;
+  using U = typename W::U;
+  constexpr int B2 = B * B, H = ilu_half(B);
+  // halves loaded together
+  constexpr int N = B == 1 ? 2 : 1;
+  constexpr unsigned kAll = 0xffffffffu;
+  const int lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+  const int g1 = A.gptr[rank + 1];
+  int g = A.gptr[rank] + int(threadIdx.x >> 5);
+  if (g >= g1)
+    return;
+  // after a round of polls: whether the warp gives up (after wait_ns, or with
+  // another warp of the CTA)
+  unsigned spins = 0;
+  unsigned long long t0 = 0;
+  auto expired = [&]() -> bool {
+    if ((++spins & 1023u) != 0)
+      return false;
+    const unsigned long long t = global_ns();
+    t0 = t0 ? t0 : t;
+    const bool end = __any_sync(kAll, *give_up || t - t0 > wait_ns);
+    if (end)
+      *give_up = 1;
+    return end;
+  };
+  int ni = __ldg(A.row + int64_t(g) * kSlice + lane);
+  int n0 = __ldg(A.base + g), n1 = __ldg(A.base + g + 1);
+  for (; g < g1; g += nw) {
+    const int i = ni, b0 = n0 >> 1, b1 = n1 >> 1;
+    const bool far = n0 & 1;
+    if (g + nw < g1) { // the next group's head, while this one waits
+      ni = __ldg(A.row + int64_t(g + nw) * kSlice + lane);
+      n0 = __ldg(A.base + g + nw);
+      n1 = __ldg(A.base + g + nw + 1);
+    }
+    T acc[B], D[UP ? B2 : 1];
+#pragma unroll
+    for (int r = 0; r < B; ++r)
+      acc[r] = i < 0 ? T(0)
+                     : (UP ? __ldcg(in + int64_t(i) * B + r) : in[int64_t(i) * B + r]);
+    if (UP) {
+#pragma unroll
+      for (int q = 0; q < B2; ++q)
+        D[q] = __ldg(A.dinv + (int64_t(g) * B2 + q) * kSlice + lane);
+    }
+    T ui[UP ? B : 1];
+    if (UP && u && !u_zero && i >= 0) {
+#pragma unroll
+      for (int r = 0; r < B; ++r)
+        ui[r] = u[int64_t(i) * B + r];
+    }
+    const uint32_t own = y + uint32_t((i - rank * A.chunk) * B) * uint32_t(sizeof(T));
+    for (int b = b0; b < b1; b += N * H) {
+      uint32_t at[N * H];
+      T m[N * H][B2];
+      const int* cp = A.col + int64_t(b) * kSlice + lane;
+      const T* vp = A.val + int64_t(b) * B2 * kSlice + lane;
+#pragma unroll
+      for (int e = 0; e < N * H; ++e)
+        if (e < H || b + H < b1) {
+          at[e] = uint32_t(__ldg(cp + e * kSlice));
+#pragma unroll
+          for (int p = 0; p < B2; ++p)
+            m[e][p] = __ldg(vp + (e * B2 + p) * kSlice);
+        }
+#pragma unroll
+      for (int e = 0; e < N * H; ++e)
+        if (e < H || b + H < b1) {
+          const uint32_t c = at[e];
+          at[e] = y + (c & uint32_t(kIluPlaceMask)) * uint32_t(sizeof(T));
+          if (far)
+            asm volatile("mapa.shared::cluster.u32 %0, %1, %2;"
+                         : "=r"(at[e]) : "r"(at[e]), "r"(c >> kIluOwnerShift));
+        }
+      auto consume = [&](auto is_far, auto half) {
+        constexpr bool kFar = decltype(is_far)::value;
+        constexpr int h = decltype(half)::value * H;
+        // what a row waits for longest is mostly its last entry: that one is
+        // polled alone (a load and a vote), then all are read
+        while (__any_sync(kAll, W::upper(W::template load<kFar>(at[h + H - 1])) ==
+                                  0xffffffffu) &&
+               !expired())
+          ;
+        U v[H][B];
+        uint32_t top;
+        do {
+#pragma unroll
+          for (int e = 0; e < H; ++e)
+#pragma unroll
+            for (int q = 0; q < B; ++q)
+              v[e][q] = W::template load<kFar>(at[h + e] + q * uint32_t(sizeof(T)));
+          uint32_t t[2] = { 0, 0 }; // two chains
+#pragma unroll
+          for (int e = 0; e < H; ++e)
+#pragma unroll
+            for (int q = 0; q < B; ++q)
+              t[(e * B + q) & 1] = max(t[(e * B + q) & 1], W::upper(v[e][q]));
+          top = max(t[0], t[1]);
+        } while (__any_sync(kAll, top == 0xffffffffu) && !expired());
+#pragma unroll
+        for (int e = 0; e < H; ++e)
+#pragma unroll
+          for (int r = 0; r < B; ++r)
+#pragma unroll
+            for (int q = 0; q < B; ++q) // before the row's first entry: 0 * 0
+              acc[r] = ilu_sub(acc[r], ilu_mul(m[h + e][r * B + q], W::value(v[e][q])));
+      };
+      using First = std::integral_constant<int, 0>;
+      using Second = std::integral_constant<int, N - 1>;
+      if (far)
+        consume(std::true_type{}, First{});
+      else
+        consume(std::false_type{}, First{});
+      if (N == 2 && b + H < b1) {
+        if (far)
+          consume(std::true_type{}, Second{});
+        else
+          consume(std::false_type{}, Second{});
+      }
+    }
+    if (UP) {
+      T z[B];
+#pragma unroll
+      for (int r = 0; r < B; ++r) {
+        z[r] = ilu_mul(D[r * B], acc[0]);
+#pragma unroll
+        for (int q = 1; q < B; ++q)
+          z[r] = ilu_add(z[r], ilu_mul(D[r * B + q], acc[q]));
+      }
+#pragma unroll
+      for (int r = 0; r < B; ++r)
+        acc[r] = z[r];
+    }
+    if (i >= 0) {
+#pragma unroll
+      for (int r = 0; r < B; ++r) {
+        const U w = W::bits(acc[r]);
+        W::store(own + r * uint32_t(sizeof(T)), W::upper(w) == 0xffffffffu ? W::kNaN : w);
+      }
+#pragma unroll
+      for (int r = 0; r < B; ++r) {
+        const int64_t k = int64_t(i) * B + r;
+        out[k] = acc[r];
+        if (UP && u) {
+          const T s = ilu_mul(omega, acc[r]);
+          u[k] = u_zero ? s : ilu_add(ui[r], s);
+        }
+      }
+    }
+    __syncwarp();
+  }
+}
+
+// h = (L U)^-1 rhs by both substitutions in one launch of one thread-block
+// cluster, then u = (u_zero ? 0 : u) + omega h (u may be null). What bounds it
+// is the chain of dependency levels (449 per direction on a 65^3 lexicographic
+// mesh), not the bytes: so y lives in the CTAs' shared memory, where a row sees
+// a dependency about 0.1 us after it was written (its own CTA's memory, or the
+// owner's over the cluster network), and rows wait for the values themselves,
+// with no barrier or launch between levels. A group's matrix entries are loaded
+// before it waits, so the other warps' loads run meanwhile. Each row runs
+// ilu_row's arithmetic in its order: the same bits. Measured on the 65^3 Q1
+// level (FP64, both substitutions): 0.65 ms against about 3.4 ms with the level
+// launches; a mixed solve of that mesh (6 steps) 112.9 -> 22.7 ms. About 0.42
+// us per level within one CTA, 0.72 us where levels cross CTAs. More warps hide
+// the matrix loads: 128 / 256 / 384 / 512 threads 1.81 / 0.98 / 0.74 / 0.65 ms
+// on the 65^3 level; two groups per average level and CTA (kIluGroupsPerLevel):
+// 1 / 2 / 4 measured 100 / 95 / 96 us on the 17^3 level, 225 / 232 / 282 us on
+// the 33^3 one. Levels whose y exceeds the cluster's shared memory (about
+// 440,000 rows in FP64, twice that in FP32) keep the level launches. Every wait
+// ends: a row
+// waits only for rows of earlier levels, a warp takes its groups in level
+// order, and the CTAs of a cluster run at the same time; bounded all the same.
+template<int B, class T>
+__global__ void __launch_bounds__(kIluClusterThreads, 1)
+k_ilu_cluster(IluPack<T> lo, IluPack<T> up, int n, const T* rhs, T* h, T* u, double omega,
+              int u_zero, int* err, unsigned long long wait_ns)
+{
+  extern __shared__ __align__(16) unsigned char ilu_smem[];
+  __shared__ int give_up;
+  using W = IluWord<T>;
+  uint32_t rank;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
+  const uint32_t y = static_cast<uint32_t>(__cvta_generic_to_shared(ilu_smem));
+  const int mine = min(lo.chunk, n - int(rank) * lo.chunk) * B;
+  auto mark = [&]() {
+    for (int k = threadIdx.x; k < mine; k += blockDim.x)
+      W::store(y + uint32_t(k) * uint32_t(sizeof(T)), W::kMark);
+  };
+  if (threadIdx.x == 0)
+    give_up = 0;
+  if (threadIdx.x < B) // what the entries before a row's first one read
+    W::store(y + uint32_t(lo.chunk * B + threadIdx.x) * uint32_t(sizeof(T)), 0);
+  mark();
+  GB_PDL_ENTRY();
+  cluster_barrier();
+  ilu_cluster_run<B, T, false>(lo, y, int(rank), rhs, h, nullptr, T(0), false, &give_up, wait_ns);
+  cluster_barrier();
+  mark();
+  cluster_barrier();
+  ilu_cluster_run<B, T, true>(up, y, int(rank), h, h, u, static_cast<T>(omega), u_zero != 0,
+                              &give_up, wait_ns);
+  cluster_barrier(); // no CTA leaves while another reads its part of y
+  if (threadIdx.x == 0 && give_up)
+    atomicExch(err, 1);
 }
 
 // u = (u_zero ? 0 : u) + omega h (StdSolver::Add after the ILU solve, unfused)

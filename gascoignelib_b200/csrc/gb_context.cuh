@@ -295,6 +295,12 @@ struct Level
     bool cta;
   };
   std::vector<IluSeg> ilu_lseg, ilu_useg;
+  // the packed factors of the cluster substitution (k_ilu_cluster), forward 0
+  // and backward 1; ctas 0: the level's rows do not fit a cluster
+  int ilu_ctas = 0, ilu_chunk = 0, ilu_groups[2] = { 0, 0 };
+  DeviceArray<int> ilu_gptr[2], ilu_grow[2], ilu_gbase[2], ilu_gcol[2];
+  DeviceArray<double> ilu_gval64[2], ilu_gdinv64;
+  DeviceArray<float> ilu_gval32[2], ilu_gdinv32;
   // values assembled on the device since the host copy was made
   bool h_val_stale = false;
   // per A^T SELL entry the A SELL entry it copies (-1: padding), block size 1:
@@ -452,6 +458,10 @@ struct gb_ctx
   // widest substitution level run inside a single-CTA launch
   // (GB_ILU_CTA_ROWS; 0: one launch per level)
   int ilu_cta_rows = gb::kIluCtaDefaultRows;
+  // substitutions in one cluster where a level fits one (off when
+  // GB_ILU_CTA_ROWS asks for the level launches)
+  bool ilu_cluster = true;
+  int ilu_max_ctas = 0; // largest cluster of k_ilu_cluster (0: not queried)
   // GB_CLUSTER=1: the levels of at most cluster_rows dofs below the finest
   // (and above the single-CTA coarse levels) as one op program run by one
   // thread-block cluster of 16 CTAs with the hardware cluster barrier between
@@ -599,6 +609,33 @@ launch_smem(Context& c, void (*kern)(KArgs...), int grid, int block, int smem,
   kt_end(c, e0, reinterpret_cast<const void*>(kern));
 }
 
+// One thread-block cluster of `ctas` blocks.
+template<class... KArgs, class... Args>
+inline void
+launch_cluster(Context& c, void (*kern)(KArgs...), int ctas, int block, int smem, Args... args)
+{
+  cudaEvent_t e0;
+  kt_begin(c, &e0);
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(ctas);
+  cfg.blockDim = dim3(block);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = c.stream;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = ctas;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = c.pdl ? 2 : 1;
+  GB_CUDA(cudaLaunchKernelEx(&cfg, kern, static_cast<KArgs>(args)...));
+  c.launches++;
+  check_launch(c);
+  kt_end(c, e0, reinterpret_cast<const void*>(kern));
+}
+
 template<class... KArgs, class... Args>
 inline void
 launch(Context& c, void (*kern)(KArgs...), int grid, int block, Args... args)
@@ -696,6 +733,15 @@ void ensure_pf_scratch(Context& c, int64_t n);
 bool direct_on(const Context& c);
 void ensure_vanka(Context& c, Level& L);
 void ensure_ilu(Context& c, Level& L);
+void ensure_wait_flag(Context& c);
+void throw_if_wait_ended(Context& c);
+// whether k_ilu_cluster runs level L's substitutions on values of T
+template<class T>
+inline bool
+ilu_in_cluster(const Context& c, const Level& L)
+{
+  return L.ilu_ctas > 0 && size_t(L.ilu_chunk) * L.B * sizeof(T) <= kIluClusterBytes;
+}
 void ensure_work(Context& c);
 
 template<int MODE, int B, class TV, class TX, class TO>

@@ -306,6 +306,41 @@ if (up) {                                                                       
 }
 
 template<class T>
+static IluPack<T>
+ilu_pack_of(const Level& L, int dir)
+{
+  const void* val = sizeof(T) == 8 ? static_cast<const void*>(L.ilu_gval64[dir].p)
+                                   : static_cast<const void*>(L.ilu_gval32[dir].p);
+  const void* dinv = sizeof(T) == 8 ? static_cast<const void*>(L.ilu_gdinv64.p)
+                                    : static_cast<const void*>(L.ilu_gdinv32.p);
+  return IluPack<T>{ L.ilu_chunk, L.ilu_gptr[dir].p, L.ilu_grow[dir].p, L.ilu_gbase[dir].p,
+                     L.ilu_gcol[dir].p, static_cast<const T*>(val),
+                     static_cast<const T*>(dinv) };
+}
+
+template<class T>
+void Emit<T>::ilu_cluster(int l, const T* rhs, T* h, T* u, bool u_zero)
+{
+  const Level& L = c.L[l];
+  no_rec();
+  auto run = [&](auto* kern) {
+    const size_t smem = (size_t(L.ilu_chunk) + 1) * L.B * sizeof(T);
+    GB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    GB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 int(kIluClusterBytes + 32)));
+    launch_cluster(c, kern, L.ilu_ctas, kIluClusterThreads, int(smem), ilu_pack_of<T>(L, 0),
+                   ilu_pack_of<T>(L, 1), (int)L.n, rhs, h, u, c.params.omega, int(u_zero),
+                   c.miderr.p, c.wait_ns);
+  };
+  switch (L.B) {
+    case 1: run(k_ilu_cluster<1, T>); break;
+    case 2: run(k_ilu_cluster<2, T>); break;
+    case 3: run(k_ilu_cluster<3, T>); break;
+    default: run(k_ilu_cluster<4, T>);
+  }
+}
+
+template<class T>
 void Emit<T>::ilu_axpy(int l, T* u, const T* h, bool u_zero)
 {
   no_rec();
@@ -480,14 +515,22 @@ smooth(Emit<T>& E, int l, int niter, T*& u, T*& tmp, const T* b, bool& u_zero)
     if (c.params.smoother == 2) {
       // linear_smooth ilu: h = y - A u (filtered), the ILU solve of h in
       // place, u += omega h, SubtractMean(u) (StdSolver::smooth)
-      if (u_zero)
-        E.copy(l, tmp, b);
-      else
+      const bool cluster = ilu_in_cluster<T>(c, L);
+      const T* h = tmp;
+      if (!u_zero)
         E.resid(l, u, tmp, b);
+      else if (cluster && !L.pf_mask)
+        h = b; // the residual of u = 0, read where it is
+      else
+        E.copy(l, tmp, b);
       if (L.pf_mask)
         E.pf_sub(l, tmp, false);
-      E.ilu_solve(l, tmp);
-      E.ilu_axpy(l, u, tmp, u_zero);
+      if (cluster) {
+        E.ilu_cluster(l, h, tmp, u, u_zero);
+      } else {
+        E.ilu_solve(l, tmp);
+        E.ilu_axpy(l, u, tmp, u_zero);
+      }
       u_zero = false;
       if (L.pf_mask)
         E.pf_sub(l, u, true);

@@ -87,6 +87,8 @@ struct Emit
   // h = ILU^-1 h in place (SparseBlockIlu::solve with the identity order: the
   // level kernels of the forward, then of the backward substitution)
   void ilu_solve(int l, T* h);
+  // h = ILU^-1 rhs and u = (u_zero ? 0 : u) + omega h by k_ilu_cluster
+  void ilu_cluster(int l, const T* rhs, T* h, T* u, bool u_zero);
   // u = (u_zero ? 0 : u) + omega h
   void ilu_axpy(int l, T* u, const T* h, bool u_zero);
   void no_rec() const;

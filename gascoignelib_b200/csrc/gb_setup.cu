@@ -769,6 +769,175 @@ ilu_levels_upload(Context& c, Level& L)
   GB_CUDA(h2d(c.stream, L.ilu_uptr_d.p, L.ilu_uptr.data(), L.ilu_uptr.size() * sizeof(int)));
 }
 
+// The flag that a bounded device wait sets when it gives up.
+void
+ensure_wait_flag(Context& c)
+{
+  if (c.miderr.n >= 1)
+    return;
+  GB_CUDA(c.miderr.alloc(1));
+  GB_CUDA(cudaMemsetAsync(c.miderr.p, 0, sizeof(int), c.stream));
+}
+
+// After a synchronisation: reports (and clears) a wait that gave up in a call
+// that returned before its kernels had run. Only the substitution clusters
+// wait in such calls.
+void
+throw_if_wait_ended(Context& c)
+{
+  if (!c.ilu_max_ctas || !c.miderr.p)
+    return;
+  int err = 0;
+  GB_CUDA(cudaMemcpy(&err, c.miderr.p, sizeof(int), cudaMemcpyDeviceToHost));
+  if (!err)
+    return;
+  GB_CUDA(cudaMemsetAsync(c.miderr.p, 0, sizeof(int), c.stream));
+  throw Error{ GB_ETIMEOUT, "a dependency wait of the block ILU gave up waiting" };
+}
+
+// CTAs of the largest cluster the device runs k_ilu_cluster with.
+static int
+ilu_max_ctas(Context& c)
+{
+  if (c.ilu_max_ctas)
+    return c.ilu_max_ctas;
+  int size = 8; // the largest portable cluster
+  auto* kern = k_ilu_cluster<1, double>;
+  if (cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) ==
+        cudaSuccess &&
+      cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           int(kIluClusterBytes + 32)) == cudaSuccess) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(kIluClusterMax);
+    cfg.blockDim = dim3(kIluClusterThreads);
+    cfg.dynamicSmemBytes = kIluClusterBytes + 32;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = kIluClusterMax;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    int n = 0;
+    if (cudaOccupancyMaxActiveClusters(&n, kern, &cfg) == cudaSuccess && n > 0)
+      size = kIluClusterMax;
+  }
+  cudaGetLastError(); // a refused query leaves no error behind
+  return c.ilu_max_ctas = size;
+}
+
+// How the level's rows are shared out among the CTAs of k_ilu_cluster, and the
+// groups of each (once per matrix structure). lev: the rows' dependency levels
+// per direction. The cluster is the smallest power of two whose shared memory
+// holds y and in which a level of average width gives each CTA at most two
+// groups.
+static void
+ilu_groups(Context& c, Level& L, const std::vector<int> (&lev)[2], const int (&nlev)[2],
+           const std::vector<int>& ptr, const std::vector<int>& col,
+           const std::vector<int>& diag)
+{
+  L.ilu_ctas = 0;
+  const int64_t n = L.n;
+  if (!c.ilu_cluster || (n + 1) * L.B >= (int64_t(1) << kIluOwnerShift))
+    return;
+  const int most = ilu_max_ctas(c);
+  auto bytes = [&](int ctas, size_t size) { return size_t((n + ctas - 1) / ctas) * L.B * size; };
+  const size_t size = bytes(most, 8) <= kIluClusterBytes ? 8 : 4;
+  if (bytes(most, size) > kIluClusterBytes)
+    return;
+  int ctas = 1;
+  while (ctas < most &&
+         (bytes(ctas, size) > kIluClusterBytes ||
+          n > int64_t(ctas) * nlev[0] * kIluGroupsPerLevel * kSlice))
+    ctas *= 2;
+  const int chunk = static_cast<int>((n + ctas - 1) / ctas), half = ilu_half(L.B);
+  for (int dir = 0; dir < 2; ++dir) {
+    // rows sorted by (owner, level), ascending within: a counting sort
+    const int nl = nlev[dir];
+    std::vector<int> off(size_t(ctas) * nl + 1, 0), at, order(n);
+    for (int64_t i = 0; i < n; ++i)
+      off[size_t(i / chunk) * nl + lev[dir][i] + 1]++;
+    for (size_t k = 0; k + 1 < off.size(); ++k)
+      off[k + 1] += off[k];
+    at.assign(off.begin(), off.end() - 1);
+    for (int64_t i = 0; i < n; ++i)
+      order[at[size_t(i / chunk) * nl + lev[dir][i]]++] = static_cast<int>(i);
+    std::vector<int> gptr(ctas + 1, 0), row, base(1, 0);
+    for (int r = 0; r < ctas; ++r) {
+      for (int q = 0; q < nl; ++q) {
+        const int k1 = off[size_t(r) * nl + q + 1];
+        for (int k = off[size_t(r) * nl + q]; k < k1; k += kSlice) {
+          int w = 0;
+          bool far = false; // an entry in another CTA's rows
+          for (int l = 0; l < kSlice; ++l) {
+            const int i = k + l < k1 ? order[k + l] : -1;
+            row.push_back(i);
+            if (i < 0)
+              continue;
+            const int b = dir ? diag[i] + 1 : ptr[i], e = dir ? ptr[i + 1] : diag[i];
+            w = std::max(w, (e - b + half - 1) / half * half);
+            if (e > b) // ascending columns: the first and the last tell
+              far = far || col[b] / chunk != r || col[e - 1] / chunk != r;
+          }
+          GB_REQUIRE(int64_t(base.back() >> 1) + w < (int64_t(1) << 30), GB_EINVAL,
+                     "ILU groups too large");
+          base.back() |= far ? 1 : 0;
+          base.push_back(((base.back() >> 1) + w) << 1);
+        }
+      }
+      gptr[r + 1] = static_cast<int>(base.size()) - 1;
+    }
+    const size_t cols = size_t(base.back() >> 1) * kSlice, B2 = size_t(L.B) * L.B;
+    L.ilu_groups[dir] = static_cast<int>(base.size()) - 1;
+    GB_CUDA(L.ilu_gptr[dir].alloc(gptr.size()));
+    GB_CUDA(L.ilu_grow[dir].alloc(row.size()));
+    GB_CUDA(L.ilu_gbase[dir].alloc(base.size()));
+    GB_CUDA(L.ilu_gcol[dir].alloc(std::max<size_t>(cols, 1)));
+    GB_CUDA(L.ilu_gval32[dir].alloc(std::max<size_t>(cols * B2, 1)));
+    if (size == 8)
+      GB_CUDA(L.ilu_gval64[dir].alloc(std::max<size_t>(cols * B2, 1)));
+    if (dir == 1) {
+      GB_CUDA(L.ilu_gdinv32.alloc(row.size() * B2));
+      if (size == 8)
+        GB_CUDA(L.ilu_gdinv64.alloc(row.size() * B2));
+    }
+    GB_CUDA(h2d(c.stream, L.ilu_gptr[dir].p, gptr.data(), gptr.size() * sizeof(int)));
+    GB_CUDA(h2d(c.stream, L.ilu_grow[dir].p, row.data(), row.size() * sizeof(int)));
+    GB_CUDA(h2d(c.stream, L.ilu_gbase[dir].p, base.data(), base.size() * sizeof(int)));
+  }
+  L.ilu_chunk = chunk;
+  L.ilu_ctas = ctas;
+}
+
+// The factors into the packed layout of k_ilu_cluster.
+static void
+ilu_pack(Context& c, Level& L)
+{
+  if (!L.ilu_ctas)
+    return;
+  ensure_wait_flag(c);
+  for (int dir = 0; dir < 2; ++dir) {
+    const int ng = L.ilu_groups[dir], nb = blocks_for(int64_t(ng) * kSlice, 256);
+    auto pack = [&](auto kern, int* col, auto* val, auto* dinv) {
+      launch(c, kern, nb, 256, ng, L.B, L.ilu_chunk, (const int*)L.ilu_grow[dir].p,
+             (const int*)L.ilu_gbase[dir].p, (const int*)L.ilu_ptr.p, (const int*)L.ilu_col.p,
+             (const int*)L.ilu_diag.p, (const double*)L.ilu_v64.p,
+             (const int*)L.ilu_gptr[dir].p, col, val, dinv);
+    };
+    int* col = L.ilu_gcol[dir].p;
+    if (dir)
+      pack(k_ilu_pack<float, true>, col, L.ilu_gval32[dir].p, L.ilu_gdinv32.p);
+    else
+      pack(k_ilu_pack<float, false>, col, L.ilu_gval32[dir].p, L.ilu_gdinv32.p);
+    if (ilu_in_cluster<double>(c, L)) {
+      if (dir)
+        pack(k_ilu_pack<double, true>, (int*)nullptr, L.ilu_gval64[dir].p, L.ilu_gdinv64.p);
+      else
+        pack(k_ilu_pack<double, false>, (int*)nullptr, L.ilu_gval64[dir].p, L.ilu_gdinv64.p);
+    }
+  }
+}
+
 void
 ilu_structure(Context& c, Level& L)
 {
@@ -822,17 +991,18 @@ ilu_structure(Context& c, Level& L)
     for (int64_t i = 0; i < n; ++i)
       rows[fill[lv[i]]++] = static_cast<int>(i);
   };
-  std::vector<int> lrows, urows;
+  std::vector<int> lrows, urows, ulev(n, 0);
   group(lev, nl, L.ilu_lptr, lrows);
   int nu = 0;
   for (int64_t i = n - 1; i >= 0; --i) {
     int m = 0;
     for (int p = diag[i] + 1; p < ptr[i + 1]; ++p)
-      m = std::max(m, lev[col[p]] + 1);
-    lev[i] = m;
+      m = std::max(m, ulev[col[p]] + 1);
+    ulev[i] = m;
     nu = std::max(nu, m + 1);
   }
-  group(lev, nu, L.ilu_uptr, urows);
+  group(ulev, nu, L.ilu_uptr, urows);
+  ilu_groups(c, L, { std::move(lev), std::move(ulev) }, { nl, nu }, ptr, col, diag);
   GB_CUDA(L.ilu_ptr.alloc(ptr.size()));
   GB_CUDA(L.ilu_col.alloc(std::max<size_t>(col.size(), 1)));
   GB_CUDA(L.ilu_diag.alloc(n));
@@ -894,6 +1064,7 @@ ensure_ilu(Context& c, Level& L)
   }
   launch(c, k_to_float, stream_blocks(nnz * B2), 256, nnz * B2, (const double*)L.ilu_v64.p,
          L.ilu_v32.p);
+  ilu_pack(c, L);
   L.ilu_ready = true;
 }
 
@@ -984,6 +1155,7 @@ ensure_ilu_host(Context& c, Level& L)
   GB_CUDA(h2d(c.stream, L.ilu_v64.p, v.data(), v.size() * sizeof(double)));
   GB_CUDA(h2d(c.stream, L.ilu_v32.p, v32.data(), v32.size() * sizeof(float)));
   ilu_levels_upload(c, L);
+  L.ilu_ctas = 0;
   L.ilu_ready = true;
   L.ilu_struct = false; // the device path rebuilds its gather map
 }
@@ -1114,8 +1286,7 @@ ensure_work(Context& c)
   }
   if (c.midbar.n < 1) {
     GB_CUDA(c.midbar.alloc(1));
-    GB_CUDA(c.miderr.alloc(1));
-    GB_CUDA(cudaMemsetAsync(c.miderr.p, 0, sizeof(int), c.stream));
+    ensure_wait_flag(c);
   }
   c.coarse_progs.clear();
   c.dense_maps.clear();
