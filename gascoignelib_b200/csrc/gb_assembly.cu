@@ -5,6 +5,55 @@
 
 namespace gb {
 
+// CTAs of the Q2 element kernels: one warp per element, two CTAs per SM at most.
+static int
+q2_blocks(int nc)
+{
+  return std::min(blocks_for(nc, kQ2Warps), 2 * 148);
+}
+
+// The element matrices of a level of patch elements (Q2, or Q1 functions on
+// patches) into asm_E, for the convection of its last assembly: plain Q2
+// elements by the matrix-unit kernel, the others by the shuffle kernel.
+static void
+patch_elements(Context& c, const Level& L, bool lps, double s0, double xeta)
+{
+  const int nc = static_cast<int>(L.mesh_ncells);
+  const double b0 = L.m_beta[0], b1 = L.m_beta[1], b2 = L.m_beta[2];
+  const bool conv = b0 != 0.0 || b1 != 0.0 || b2 != 0.0;
+  const double bnorm = std::sqrt(b0 * b0 + b1 * b1 + b2 * b2) + 1e-6;
+  const double g = 0.5 / std::sqrt(3.0);
+  auto plain = [&](auto* kern, size_t smem) {
+    GB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+    launch_smem(c, kern, q2_blocks(nc), 32 * kQ2Warps, int(smem), nc, (const int*)L.m_cells.p,
+                (const double*)L.m_coords.p, (const double*)L.m_kappa.p, b0, b1, b2, c.asm_E.p);
+  };
+  auto shuffled = [&](auto* kern) {
+    launch(c, kern, blocks_for(int64_t(nc) * 32, 128), 128, nc, (const int*)L.m_cells.p,
+           (const double*)L.m_coords.p, (const double*)L.m_kappa.p, b0, b1, b2, c.asm_E.p, s0,
+           xeta, bnorm, g);
+  };
+  if (L.mesh_deg == 2 && !lps) {
+    if (L.mesh_dim == 2)
+      plain(conv ? k_q2_element<2, true> : k_q2_element<2, false>, q2_smem<2>());
+    else
+      plain(conv ? k_q2_element<3, true> : k_q2_element<3, false>, q2_smem<3>());
+  } else if (L.mesh_deg == 2) {
+    if (L.mesh_dim == 2)
+      shuffled(k_q2_element_warp<2, true, true, false>);
+    else
+      shuffled(k_q2_element_warp<3, true, true, false>);
+  } else if (L.mesh_dim == 2) {
+    shuffled(lps    ? k_q2_element_warp<2, true, true, true>
+             : conv ? k_q2_element_warp<2, true, false, true>
+                    : k_q2_element_warp<2, false, false, true>);
+  } else {
+    shuffled(lps    ? k_q2_element_warp<3, true, true, true>
+             : conv ? k_q2_element_warp<3, true, false, true>
+                    : k_q2_element_warp<3, false, false, true>);
+  }
+}
+
 // Element matrices and their sum into level l's values (FP64 and FP32), the
 // Dirichlet rows and columns, and the block-diagonal inverse; the kappa of the
 // level's cells is in L.m_kappa.
@@ -15,7 +64,6 @@ assemble_level(Context& c, int l, const double* beta)
   const int dim = L.mesh_dim;
   const int nl = L.mesh_deg == 1 ? 1 << dim : (dim == 3 ? 27 : 9);
   const int nc = static_cast<int>(L.mesh_ncells);
-  const bool pq1 = L.mesh_deg == 3; // Q1 functions on patches
   GB_CUDA(c.asm_E.n >= size_t(nc) * nl * nl ? cudaSuccess
                                              : c.asm_E.alloc(size_t(nc) * nl * nl));
   const double b0 = beta ? beta[0] : 0.0, b1 = beta ? beta[1] : 0.0;
@@ -31,34 +79,17 @@ assemble_level(Context& c, int l, const double* beta)
 #define GB_ELEM(D, CV)                                                                   \
   launch(c, k_q1_element<D, CV>, blocks_for(nc, 128), 128, nc, (const int*)L.m_cells.p,  \
          (const double*)L.m_coords.p, (const double*)L.m_kappa.p, b0, b1, b2, g, c.asm_E.p)
-#define GB_ELEM2(D, CV, LP, PQ)                                                          \
-  launch(c, k_q2_element_warp<D, CV, LP, PQ>, blocks_for(int64_t(nc) * 32, 128), 128, nc, \
-         (const int*)L.m_cells.p, (const double*)L.m_coords.p, (const double*)L.m_kappa.p, \
-         b0, b1, b2, c.asm_E.p, c.lps_s0, c.lps_xeta, bnorm, g)
-#define GB_ELEM2K(D, PQ)                                                                 \
-  do {                                                                                   \
-    if (lps) GB_ELEM2(D, true, true, PQ);                                                \
-    else if (conv) GB_ELEM2(D, true, false, PQ);                                         \
-    else GB_ELEM2(D, false, false, PQ);                                                  \
-  } while (0)
   GB_REQUIRE(c.lps_s0 == 0.0 || L.mesh_deg >= 2, GB_EINVAL,
              "LPS is built for patch elements only (Q2, or Q1 on patches)");
   const bool lps = conv && c.lps_s0 > 0.0;
-  const double bnorm = std::sqrt(b0 * b0 + b1 * b1 + b2 * b2) + 1e-6;
   if (L.mesh_deg >= 2) {
-    if (dim == 2) {
-      if (pq1) GB_ELEM2K(2, true); else GB_ELEM2K(2, false);
-    } else {
-      if (pq1) GB_ELEM2K(3, true); else GB_ELEM2K(3, false);
-    }
+    patch_elements(c, L, lps, c.lps_s0, c.lps_xeta);
   } else if (dim == 2) {
     if (conv) GB_ELEM(2, true); else GB_ELEM(2, false);
   } else {
     if (conv) GB_ELEM(3, true); else GB_ELEM(3, false);
   }
 #undef GB_ELEM
-#undef GB_ELEM2
-#undef GB_ELEM2K
   if (L.m_nhcells > 0)
     launch(c, k_condense, blocks_for(int64_t(L.m_nhcells) * 32, 128), 128, L.m_nhcells,
            (const int*)L.m_hcells.p, (const int*)L.m_hopptr.p, (const CondOp*)L.m_hops.p, nl,
@@ -163,32 +194,28 @@ form_level(Context& c, int l, double* y, double* x, double d)
       if (conv) GB_FORM(3, true); else GB_FORM(3, false);
     }
 #undef GB_FORM
+  } else if (L.mesh_deg == 2 && !(conv && L.m_lps_s0 > 0.0)) {
+    auto form = [&](auto* kern, size_t smem) {
+      GB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+      launch_smem(c, kern, q2_blocks(nc), 32 * kQ2Warps, int(smem), nc,
+                  (const int*)L.m_cells.p, (const double*)L.m_coords.p,
+                  (const double*)L.m_kappa.p, b0, b1, b2, (const double*)x, c.asm_R.p);
+    };
+    if (dim == 2)
+      form(conv ? k_q2_form<2, true> : k_q2_form<2, false>, q2_smem<2>());
+    else
+      form(conv ? k_q2_form<3, true> : k_q2_form<3, false>, q2_smem<3>());
   } else {
     GB_CUDA(c.asm_E.n >= size_t(nc) * nl * nl ? cudaSuccess
                                                : c.asm_E.alloc(size_t(nc) * nl * nl));
-    const bool pq1 = L.mesh_deg == 3, lps = conv && L.m_lps_s0 > 0.0;
-    const double bnorm = std::sqrt(b0 * b0 + b1 * b1 + b2 * b2) + 1e-6;
-#define GB_ELEM2(D, CV, LP, PQ)                                                          \
-  launch(c, k_q2_element_warp<D, CV, LP, PQ>, blocks_for(int64_t(nc) * 32, 128), 128, nc, \
-         (const int*)L.m_cells.p, (const double*)L.m_coords.p, (const double*)L.m_kappa.p, \
-         b0, b1, b2, c.asm_E.p, L.m_lps_s0, L.m_lps_xeta, bnorm, g)
-#define GB_ELEM2K(D, PQ)                                                                 \
-  do {                                                                                   \
-    if (lps) GB_ELEM2(D, true, true, PQ);                                                \
-    else if (conv) GB_ELEM2(D, true, false, PQ);                                         \
-    else GB_ELEM2(D, false, false, PQ);                                                  \
-  } while (0)
-    if (dim == 2) {
-      if (pq1) GB_ELEM2K(2, true); else GB_ELEM2K(2, false);
-      launch(c, k_elem_apply<9>, blocks_for(int64_t(nc) * 32, 128), 128, nc,
-             (const int*)L.m_cells.p, (const double*)c.asm_E.p, (const double*)x, c.asm_R.p);
-    } else {
-      if (pq1) GB_ELEM2K(3, true); else GB_ELEM2K(3, false);
-      launch(c, k_elem_apply<27>, blocks_for(int64_t(nc) * 32, 128), 128, nc,
-             (const int*)L.m_cells.p, (const double*)c.asm_E.p, (const double*)x, c.asm_R.p);
-    }
-#undef GB_ELEM2
-#undef GB_ELEM2K
+    patch_elements(c, L, conv && L.m_lps_s0 > 0.0, L.m_lps_s0, L.m_lps_xeta);
+    const int nb = blocks_for(int64_t(nc) * 32, 128);
+    if (dim == 2)
+      launch(c, k_elem_apply<9>, nb, 128, nc, (const int*)L.m_cells.p,
+             (const double*)c.asm_E.p, (const double*)x, c.asm_R.p);
+    else
+      launch(c, k_elem_apply<27>, nb, 128, nc, (const int*)L.m_cells.p,
+             (const double*)c.asm_E.p, (const double*)x, c.asm_R.p);
   }
   launch(c, k_form_gather, blocks_for(L.n, 256), 256, (int)L.n, (const int*)L.m_nptr.p,
          (const int*)L.m_nlist.p, (const double*)c.asm_R.p, d, y);

@@ -364,6 +364,309 @@ k_q2_element_warp(int ncells, const int* __restrict__ cells,
   }
 }
 
+// ------------------------------------------------ Q2 elements, plain equation
+//
+// The element matrix as a contraction over the Gauss points. With the
+// reference gradients D_k(a, q) of the 3^DIM functions (the same for every
+// element) and, per point, the metric M_q = w |J| kappa J^-1 J^-T and the row
+// c_q = w |J| beta J^-T,
+//   E(a, b) = sum_q sum_k D_k(a, q) (M_q D(b, q))_k + phi_a(q) (c_q . D(b, q)),
+// a product of inner length 4 per point (3 metric rows and the convection's).
+// One warp per element: lane q first forms point q's J, M_q and c_q, then the
+// warp multiplies on the FP64 matrix unit (mma m8n8k4: the tables' entries are
+// one operand, and a lane forms its entries of the other from its row of
+// (M_q, c_q)), 4 x 4 tiles of 8 x 8 in 2 x 16 accumulators per lane (27 of 32
+// rows and columns used). The tables stay in shared memory for all elements of
+// a CTA. What bounds it is the FP64 unit (432 products of 8 x 8 x 4 per element,
+// 1.4 times the useful multiply-adds). Measured on 32,768
+// elements and their coarser levels: 0.54 ms, against 3.2 ms for the form with
+// a warp per element that passed the gradients by shuffles (k_q2_element_warp,
+// kept for LPS and for Q1 functions on patches).
+template<int DIM>
+struct Q2Tab
+{
+  static constexpr int NL = DIM == 3 ? 27 : 9; // nodes, and Gauss points
+  static constexpr int MT = (NL + 7) / 8;      // 8-wide tiles
+  static constexpr int CS = MT * 8 + 4;        // table stride per component (bank-free)
+  static constexpr int QS = 4 * CS + 1;        // and per point (odd: lane = point)
+  static constexpr int NS = 13;                // per-point (M, c) stride
+  static constexpr int kWarp = NL * NS + NL * DIM + (DIM == 3 ? 0 : 1); // per-warp doubles
+};
+constexpr int kQ2Warps = 8;
+template<int DIM>
+constexpr size_t
+q2_smem()
+{
+  return (size_t(Q2Tab<DIM>::NL) * Q2Tab<DIM>::QS + size_t(kQ2Warps) * Q2Tab<DIM>::kWarp) *
+         sizeof(double);
+}
+
+// tab[q QS + k CS + a]: D_k(a, q) for k < DIM, phi_a(q) for k = 3, else 0.
+template<int DIM>
+__device__ __forceinline__ void
+q2_table(double* tab)
+{
+  using Q = Q2Tab<DIM>;
+  const double P3[3] = { 0.11270166537925831148, 0.5, 0.88729833462074168852 };
+  for (int e = threadIdx.x; e < Q::NL * 4 * Q::MT * 8; e += blockDim.x) {
+    const int a = e % (Q::MT * 8), k = (e / (Q::MT * 8)) % 4, q = e / (Q::MT * 32);
+    double v = a < Q::NL && (k < DIM || k == 3) ? 1.0 : 0.0;
+    int ad = a, qd = q;
+#pragma unroll
+    for (int d = 0; d < DIM; ++d) {
+      const double t = qd % 3 == 0 ? P3[0] : qd % 3 == 1 ? P3[1] : P3[2];
+      double L[3], dL[3];
+      q2_basis_1d(t, L, dL);
+      const int i = ad % 3;
+      const double l = i == 0 ? L[0] : i == 1 ? L[1] : L[2];
+      const double g = i == 0 ? dL[0] : i == 1 ? dL[1] : dL[2];
+      v *= d == k ? g : l;
+      ad /= 3;
+      qd /= 3;
+    }
+    tab[q * Q::QS + k * Q::CS + a] = v;
+  }
+}
+
+// Lane q's (M_q, c_q) as 4 rows of DIM (row 2 of a 2D element is zero); X: the
+// element's nodes, xs (or null): nodal values, whose reference gradient at the
+// point goes to gu.
+template<int DIM, bool CONV, bool GRAD>
+__device__ __forceinline__ void
+q2_point(const double* tab, const double* X, int q, double kap, const double* beta,
+         double (&N)[4][DIM], const double* xs, double (&gu)[DIM])
+{
+  using Q = Q2Tab<DIM>;
+  const double W3[3] = { 0.277777777778, 0.444444444444, 0.277777777778 };
+  double J[DIM][DIM], wq = 1.0;
+  int qd = q;
+#pragma unroll
+  for (int d = 0; d < DIM; ++d) {
+    wq *= qd % 3 == 1 ? W3[1] : W3[0];
+    qd /= 3;
+    gu[d] = 0.0;
+#pragma unroll
+    for (int k = 0; k < DIM; ++k)
+      J[d][k] = 0.0;
+  }
+#pragma unroll 3
+  for (int b = 0; b < Q::NL; ++b) {
+    double g[DIM];
+#pragma unroll
+    for (int k = 0; k < DIM; ++k)
+      g[k] = tab[q * Q::QS + k * Q::CS + b];
+#pragma unroll
+    for (int d = 0; d < DIM; ++d) {
+      const double x = X[b * DIM + d];
+#pragma unroll
+      for (int k = 0; k < DIM; ++k)
+        J[d][k] = fma(x, g[k], J[d][k]);
+    }
+    if (GRAD) {
+      const double u = xs[b];
+#pragma unroll
+      for (int k = 0; k < DIM; ++k)
+        gu[k] = fma(u, g[k], gu[k]);
+    }
+  }
+  double det, Ji[DIM][DIM];
+  if (DIM == 2) {
+    det = J[0][0] * J[1][1] - J[0][1] * J[1][0];
+    const double r = 1.0 / det;
+    Ji[0][0] = J[1][1] * r;
+    Ji[0][1] = -J[0][1] * r;
+    Ji[1][0] = -J[1][0] * r;
+    Ji[1][1] = J[0][0] * r;
+  } else {
+    const double c00 = J[1][1] * J[2][2] - J[1][2] * J[2][1];
+    const double c01 = J[1][2] * J[2][0] - J[1][0] * J[2][2];
+    const double c02 = J[1][0] * J[2][1] - J[1][1] * J[2][0];
+    det = J[0][0] * c00 + J[0][1] * c01 + J[0][2] * c02;
+    const double r = 1.0 / det;
+    Ji[0][0] = c00 * r;
+    Ji[1][0] = c01 * r;
+    Ji[2][0] = c02 * r;
+    Ji[0][1] = (J[0][2] * J[2][1] - J[0][1] * J[2][2]) * r;
+    Ji[1][1] = (J[0][0] * J[2][2] - J[0][2] * J[2][0]) * r;
+    Ji[2][1] = (J[0][1] * J[2][0] - J[0][0] * J[2][1]) * r;
+    Ji[0][2] = (J[0][1] * J[1][2] - J[0][2] * J[1][1]) * r;
+    Ji[1][2] = (J[0][2] * J[1][0] - J[0][0] * J[1][2]) * r;
+    Ji[2][2] = (J[0][0] * J[1][1] - J[0][1] * J[1][0]) * r;
+  }
+  const double w = wq * fabs(det), wk = w * kap;
+#pragma unroll
+  for (int l = 0; l < DIM; ++l) {
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      double m = 0.0;
+      if (k < DIM) {
+#pragma unroll
+        for (int d = 0; d < DIM; ++d)
+          m = fma(Ji[k < DIM ? k : 0][d], Ji[l][d], m);
+      }
+      N[k][l] = wk * m;
+    }
+    double s = 0.0;
+    if (CONV) {
+#pragma unroll
+      for (int d = 0; d < DIM; ++d)
+        s = fma(beta[d], Ji[l][d], s);
+    }
+    N[3][l] = w * s;
+  }
+}
+
+__device__ __forceinline__ void
+mma_f64(double (&c)[2], double a, double b)
+{
+  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+               : "+d"(c[0]), "+d"(c[1])
+               : "d"(a), "d"(b));
+}
+
+template<int DIM, bool CONV>
+__global__ void __launch_bounds__(32 * kQ2Warps, 2)
+k_q2_element(int ncells, const int* __restrict__ cells, const double* __restrict__ coords,
+             const double* __restrict__ kappa, double b0, double b1, double b2,
+             double* __restrict__ E)
+{
+  using Q = Q2Tab<DIM>;
+  extern __shared__ double q2_sm[];
+  double* tab = q2_sm;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  double* Nw = q2_sm + Q::NL * Q::QS + warp * Q::kWarp;
+  double* X = Nw + Q::NL * Q::NS;
+  q2_table<DIM>(tab);
+  GB_PDL_ENTRY();
+  __syncthreads();
+  const double beta[3] = { b0, b1, b2 };
+  const int k = lane & 3, r = lane >> 2; // the operands' inner index and row
+  for (int64_t c = int64_t(blockIdx.x) * kQ2Warps + warp; c < ncells;
+       c += int64_t(gridDim.x) * kQ2Warps) {
+    if (lane < Q::NL) {
+      const int64_t node = __ldg(cells + int64_t(lane) * ncells + c);
+#pragma unroll
+      for (int d = 0; d < DIM; ++d)
+        X[lane * DIM + d] = __ldg(coords + node * DIM + d);
+    }
+    const double kap = __ldg(kappa + c);
+    __syncwarp();
+    if (lane < Q::NL) {
+      double N[4][DIM], gu[DIM];
+      q2_point<DIM, CONV, false>(tab, X, lane, kap, beta, N, nullptr, gu);
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int l = 0; l < DIM; ++l)
+          Nw[lane * Q::NS + i * DIM + l] = N[i][l];
+    }
+    __syncwarp();
+    // without convection the matrix is symmetric: the upper tiles only
+    double acc[Q::MT][Q::MT][2];
+#pragma unroll
+    for (int i = 0; i < Q::MT; ++i)
+#pragma unroll
+      for (int j = 0; j < Q::MT; ++j)
+        acc[i][j][0] = acc[i][j][1] = 0.0;
+#pragma unroll 1
+    for (int q = 0; q < Q::NL; ++q) {
+      const double* t = tab + q * Q::QS + r;
+      double n[DIM], a[Q::MT], b[Q::MT];
+#pragma unroll
+      for (int l = 0; l < DIM; ++l)
+        n[l] = Nw[q * Q::NS + k * DIM + l];
+#pragma unroll
+      for (int i = 0; i < Q::MT; ++i) {
+        a[i] = t[k * Q::CS + i * 8];
+        double s = 0.0;
+#pragma unroll
+        for (int l = 0; l < DIM; ++l)
+          s = fma(n[l], t[l * Q::CS + i * 8], s);
+        b[i] = s;
+      }
+#pragma unroll
+      for (int i = 0; i < Q::MT; ++i)
+#pragma unroll
+        for (int j = CONV ? 0 : i; j < Q::MT; ++j)
+          mma_f64(acc[i][j], a[i], b[j]);
+    }
+    __syncwarp();
+#pragma unroll
+    for (int i = 0; i < Q::MT; ++i)
+#pragma unroll
+      for (int j = CONV ? 0 : i; j < Q::MT; ++j)
+#pragma unroll
+        for (int p = 0; p < 2; ++p) {
+          const int row = i * 8 + r, col = j * 8 + 2 * k + p;
+          if (row < Q::NL && col < Q::NL) {
+            E[(int64_t(row) * Q::NL + col) * ncells + c] = acc[i][j][p];
+            if (!CONV && j > i)
+              E[(int64_t(col) * Q::NL + row) * ncells + c] = acc[i][j][p];
+          }
+        }
+  }
+}
+
+// The element residuals of the same equation, without its matrices: with the
+// reference gradient g_q of x at point q,
+//   R(a) = sum_q sum_k D_k(a, q) (M_q g_q)_k + phi_a(q) (c_q . g_q).
+// One warp per element, lane = point for the first part, lane = node for the
+// second: 2 x 3^DIM short products instead of the 3^DIM x 3^DIM matrix.
+template<int DIM, bool CONV>
+__global__ void __launch_bounds__(32 * kQ2Warps, 2)
+k_q2_form(int ncells, const int* __restrict__ cells, const double* __restrict__ coords,
+          const double* __restrict__ kappa, double b0, double b1, double b2,
+          const double* __restrict__ x, double* __restrict__ R)
+{
+  using Q = Q2Tab<DIM>;
+  extern __shared__ double q2_sm[];
+  double* tab = q2_sm;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  double* Tw = q2_sm + Q::NL * Q::QS + warp * Q::kWarp; // 4 per point, then x
+  double* xs = Tw + Q::NL * 4;
+  double* X = Tw + Q::NL * Q::NS;
+  q2_table<DIM>(tab);
+  GB_PDL_ENTRY();
+  __syncthreads();
+  const double beta[3] = { b0, b1, b2 };
+  for (int64_t c = int64_t(blockIdx.x) * kQ2Warps + warp; c < ncells;
+       c += int64_t(gridDim.x) * kQ2Warps) {
+    if (lane < Q::NL) {
+      const int64_t node = __ldg(cells + int64_t(lane) * ncells + c);
+      xs[lane] = __ldg(x + node);
+#pragma unroll
+      for (int d = 0; d < DIM; ++d)
+        X[lane * DIM + d] = __ldg(coords + node * DIM + d);
+    }
+    const double kap = __ldg(kappa + c);
+    __syncwarp();
+    if (lane < Q::NL) {
+      double N[4][DIM], gu[DIM];
+      q2_point<DIM, CONV, true>(tab, X, lane, kap, beta, N, xs, gu);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        double s = 0.0;
+#pragma unroll
+        for (int l = 0; l < DIM; ++l)
+          s = fma(N[i][l], gu[l], s);
+        Tw[lane * 4 + i] = s;
+      }
+    }
+    __syncwarp();
+    if (lane < Q::NL) {
+      double s = 0.0;
+#pragma unroll 3
+      for (int q = 0; q < Q::NL; ++q)
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+          if (i < DIM || (CONV && i == 3))
+            s = fma(tab[q * Q::QS + i * Q::CS + lane], Tw[q * 4 + i], s);
+      R[int64_t(lane) * ncells + c] = s;
+    }
+    __syncwarp();
+  }
+}
+
 // One step of the hanging-node condensation of an element matrix: with t >= 0
 // column t += w column s, then row t += w row s (a parent of the hanging node
 // in slot s that the element holds in slot t); with t < 0 column s and row s
