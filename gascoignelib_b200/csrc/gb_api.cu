@@ -33,6 +33,8 @@ gb_ctx_create(gb_ctx** out, int device)
       ctx->row_order = atoi(e) != 0;
     if (const char* e = getenv("GB_ILU_CTA_ROWS"))
       ctx->ilu_cta_rows = std::max(0, atoi(e)), ctx->ilu_cluster = false;
+    if (const char* e = getenv("GB_EXACT_CTAS"))
+      ctx->exact_ctas = std::min(std::max(0, atoi(e)), kExactMaxCtas);
     if (const char* e = getenv("GB_VANKA_HOST"))
       ctx->vanka_host = atoi(e) != 0;
     if (const char* e = getenv("GB_CLUSTER"))

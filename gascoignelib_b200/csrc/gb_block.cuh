@@ -1031,7 +1031,6 @@ k_ilu_pack(int ngroups, int B, int chunk, const int* __restrict__ row,
 constexpr int kIluClusterThreads = 512;
 constexpr size_t kIluClusterBytes = 216 * 1024; // of y in a CTA's shared memory
 constexpr int kIluGroupsPerLevel = 2;           // a CTA's share of an average level
-constexpr int kIluClusterMax = 16;              // CTAs (16: not a portable size)
 
 // One direction of k_ilu_cluster: this CTA's groups, warp by warp in level
 // order. in: the rows' right-hand side; out: the result in global memory. All

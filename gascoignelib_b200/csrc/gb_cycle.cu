@@ -365,6 +365,37 @@ void Emit<T>::jacobi(int l, const T* u, T* out, const T* b)
 }
 
 template<class T>
+bool Emit<T>::exact_sweeps(int l, int niter, T* u, const T* b, bool u_zero)
+{
+  const Level& L = c.L[l];
+  const Sell& A = opA(c, L);
+  // Levels up to kCoarseMaxRows have their dense map or op program; two sweeps
+  // are not worth the copy of the matrix.
+  if (rec || L.B != 1 || L.n <= kCoarseMaxRows || L.n > 65535 || niter < 3)
+    return false;
+  const int ctas = c.exact_ctas;
+  if (ctas <= 0)
+    return false;
+  const int slices = blocks_for(A.nslices, ctas);
+  if (slices > kExactWarps)
+    return false;
+  const int parts = std::min(8, kExactWarps / slices);
+  int entries = 0; // of the fullest CTA
+  for (int s = 0; s < A.nslices; s += slices)
+    entries = std::max(entries, A.h_sptr[std::min<int>(s + slices, A.nslices)] - A.h_sptr[s]);
+  const size_t smem = exact_smem<T>(L.n, entries, slices, parts);
+  if (smem > kExactBytes)
+    return false;
+  GB_CUDA(cudaFuncSetAttribute(k_exact_sweeps<T>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+  GB_CUDA(cudaFuncSetAttribute(k_exact_sweeps<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               int(kExactBytes)));
+  launch_cluster(c, k_exact_sweeps<T>, ctas, kExactWarps * 32, int(smem),
+                 view<T>(A, sell_vals<T>(A)), slices, parts, niter, int(u_zero), b,
+                 dinv_of<T>(L), u, c.params.omega, c.miderr.p, c.wait_ns);
+  return true;
+}
+
+template<class T>
 void Emit<T>::resid(int l, const T* u, T* out, const T* b)
 {
   const Level& L = c.L[l];
@@ -591,6 +622,20 @@ smooth(Emit<T>& E, int l, int niter, T*& u, T*& tmp, const T* b, bool& u_zero)
     if (L.pf_mask)
       E.pf_sub(l, u, true);
   }
+}
+
+// smooth_exact on the coarsest level (iterexact sweeps where it is not solved
+// directly): in one launch where the level below others fits a cluster.
+template<class T>
+static void
+smooth_exact(Emit<T>& E, int l, int finelevel, int niter, T*& u, T*& tmp, const T* b,
+             bool& u_zero)
+{
+  if (l < finelevel && fused_smoother(E.c, E.c.L[l]) && E.exact_sweeps(l, niter, u, b, u_zero)) {
+    u_zero = false;
+    return;
+  }
+  smooth<T>(E, l, niter, u, tmp, b, u_zero);
 }
 
 template<class T>
@@ -1028,7 +1073,7 @@ mgstep(Emit<T>& E, MgWork<T>& W, int l, int finelevel, int coarselevel, char& p0
     if (l == coarselevel) {
       if (p == 'F')
         p0 = 'V';
-      smooth<T>(E, l, P.iterexact - 1, u, tmp, b, z); // smooth_exact
+      smooth_exact<T>(E, l, finelevel, P.iterexact - 1, u, tmp, b, z);
       return false;
     }
     smooth<T>(E, l, P.iterpre - 1, u, tmp, b, z);
@@ -1049,7 +1094,7 @@ mgstep(Emit<T>& E, MgWork<T>& W, int l, int finelevel, int coarselevel, char& p0
       E.direct(l, u, b);
       return false;
     }
-    smooth<T>(E, l, P.iterexact, u, tmp, b, u_zero); // smooth_exact
+    smooth_exact<T>(E, l, finelevel, P.iterexact, u, tmp, b, u_zero);
     return u_zero;
   }
   smooth<T>(E, l, P.iterpre, u, tmp, b, u_zero);

@@ -97,6 +97,9 @@ struct Emit
   static T* vk_out(const Level& L);
   void jacobi(int l, const T* u, T* out, const T* b);
   void resid(int l, const T* u, T* out, const T* b);
+  // niter sweeps of the coarsest level in one cluster, u in place (u_zero: from
+  // 0); false where the level does not fit one
+  bool exact_sweeps(int l, int niter, T* u, const T* b, bool u_zero);
   // coarse (level l) = R fine, 0 on the coarse Dirichlet dofs; with smean
   // (block levels) the filtered component of fine is read minus *smean; with
   // u1 (scalar levels) the restriction also writes the coarse level's first

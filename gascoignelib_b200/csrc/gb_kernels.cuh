@@ -1819,6 +1819,168 @@ cluster_barrier()
                  : "memory");
 }
 
+// niter damped Jacobi sweeps x += omega D^-1 (b - A x) of a small scalar level
+// (the coarsest level's iterexact sweeps) in one launch of one cluster. A sweep
+// of a few thousand rows as a launch of its own is latency only (launch, then
+// range, column and x one after the other: 8 to 17 us for 3,375 rows of 27 or
+// 1,331 rows of up to 125 entries). Here each CTA copies its slices (`slices`
+// each) to shared memory once, with 16-bit columns, and keeps all of x; after a
+// sweep each CTA sends its new values into every CTA's copy over the cluster
+// network, each store counted on the receiver's mbarrier, and a sweep starts
+// when all n values of the last one have come (a cluster barrier per sweep
+// instead: 2 us more for 9 sweeps). Measured on 16 CTAs, 9 sweeps with events
+// around the launch: 27 us for 1,331 Q2 rows in FP32, 37 us in FP64, 25 us for
+// 3,375 Q1 rows in FP64; 8 CTAs 6 to 8 us more. Solves of 80^3 Q2 cells 51.1 ->
+// 46.3 ms, 40^3 Q2 cells with a refined ball 51.9 -> 46.6 ms, 56^3 Q1 cells
+// (left) 2.32 -> 2.28 ms. Two copies and two mbarriers take turns: a CTA
+// sends sweep k + 2 only after it has every CTA's k + 1, which that CTA sent
+// after its last read of k's copy and after its wait for k. `parts`
+// warps share a slice: each takes every parts-th entry of its 32 rows, and a
+// row's partial sums are added in the warps' order, so the order is not the
+// sequential kernel's. x holds the start (zero: from 0, the first sweep needs
+// no product) and receives the result.
+constexpr int kExactWarps = 32;
+constexpr int kExactMaxCtas = 16;
+constexpr size_t kExactBytes = 220 * 1024; // shared memory per CTA
+
+// x twice, the partial sums, the entries' values and columns
+template<class T>
+inline size_t
+exact_smem(int64_t n, int64_t entries, int slices, int parts)
+{
+  return size_t(2 * (n + (n & 1)) + int64_t(slices) * parts * kSlice) * sizeof(T) +
+         size_t(entries) * (sizeof(T) + 2);
+}
+
+// The value v to shared address a of CTA r, counted on that CTA's mbarrier.
+template<class T>
+__device__ __forceinline__ void
+send_counted(uint32_t a, uint32_t mbar, uint32_t r, T v)
+{
+  uint32_t ra, rm;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(ra) : "r"(a), "r"(r));
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(rm) : "r"(mbar), "r"(r));
+  if (sizeof(T) == 8)
+    asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.b64 [%0], %1, [%2];"
+                 ::"r"(ra), "l"(__double_as_longlong(double(v))), "r"(rm) : "memory");
+  else
+    asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.b32 [%0], %1, [%2];"
+                 ::"r"(ra), "r"(__float_as_uint(float(v))), "r"(rm) : "memory");
+}
+
+template<class T>
+__global__ void __launch_bounds__(kExactWarps * 32, 1)
+k_exact_sweeps(SellView<T> A, int slices, int parts, int niter, int zero,
+               const T* __restrict__ b, const T* __restrict__ dinv, T* __restrict__ x,
+               double omega_, int* err, unsigned long long wait_ns)
+{
+  extern __shared__ __align__(16) unsigned char exact_sm[];
+  __shared__ __align__(8) unsigned long long came[2];
+  constexpr int kThreads = kExactWarps * 32;
+  const int n = A.n, np = n + (n & 1), nsl = (n + kSlice - 1) / kSlice;
+  uint32_t rank, ctas;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
+  asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(ctas));
+  const int s0 = min(int(rank) * slices, nsl), s1 = min(s0 + slices, nsl);
+  T* xs = reinterpret_cast<T*>(exact_sm);
+  T* part = xs + 2 * np;
+  T* val = part + slices * parts * kSlice;
+  GB_PDL_ENTRY();
+  const int e0 = A.sptr[s0], ne = A.sptr[s1] - e0;
+  uint16_t* col = reinterpret_cast<uint16_t*>(val + ne);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  // this warp's (slice, part): entries j = pt, pt + parts, ... of its rows
+  const int ws = s0 + warp / parts, pt = warp % parts;
+  const bool work = ws < s1 && warp < slices * parts;
+  int beg = 0, w = 0;
+  if (work) {
+    const int slot = ws * kSlice + lane;
+    const int row = slot >= n ? 0 : A.perm ? __ldg(A.perm + slot) : slot;
+    beg = A.sptr[ws];
+    w = (A.sptr[ws + 1] - beg) >> 5;
+    const int* cp = A.pid ? A.ptab + int(A.pid[row]) * A.W : nullptr;
+#pragma unroll 4
+    for (int j = pt; j < w; j += parts) {
+      const int at = beg + j * kSlice + lane;
+      val[at - e0] = __ldg(A.val + at);
+      // past a row's end (value 0) any column will do
+      const int cj = cp ? row + __ldg(cp + j) : __ldg(A.col + at);
+      col[at - e0] = static_cast<uint16_t>(min(max(cj, 0), n - 1));
+    }
+  }
+  // this thread's row of the update, and the CTAs it sends the new value to
+  const int rows = slices * kSlice, share = kThreads / rows;
+  const int rt = threadIdx.x % rows, sub = threadIdx.x / rows;
+  const int uslot = s0 * kSlice + rt;
+  const bool upd = sub < share && uslot < min(s1 * kSlice, n);
+  const T omega = static_cast<T>(omega_);
+  int urow = 0;
+  T br = T(0), dr = T(0);
+  if (upd) {
+    urow = A.perm ? __ldg(A.perm + uslot) : uslot;
+    br = __ldg(b + urow);
+    dr = __ldg(dinv + urow);
+  }
+  for (int i = threadIdx.x; i < n; i += kThreads)
+    xs[i] = zero ? omega * (__ldg(dinv + i) * __ldg(b + i)) : x[i];
+  const uint32_t bar = static_cast<uint32_t>(__cvta_generic_to_shared(came));
+  if (threadIdx.x == 0) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar));
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar + 8));
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  cluster_barrier(); // every CTA has read x, and is there to be written to
+  const uint32_t xbase = static_cast<uint32_t>(__cvta_generic_to_shared(xs));
+  int cur = 0, turn = 0;
+  for (int it = zero ? 1 : 0; it < niter; ++it, ++turn) {
+    const uint32_t mbar = bar + 8 * (turn & 1);
+    if (threadIdx.x == 0)
+      asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;"
+                   ::"r"(mbar), "r"(uint32_t(n) * uint32_t(sizeof(T))) : "memory");
+    const T* xo = xs + cur * np;
+    if (work) {
+      T acc = T(0);
+      const T* vp = val + (beg - e0) + lane;
+      const uint16_t* cp = col + (beg - e0) + lane;
+#pragma unroll 4
+      for (int j = pt; j < w; j += parts)
+        acc = fma(vp[j * kSlice], xo[cp[j * kSlice]], acc);
+      part[warp * kSlice + lane] = acc;
+    }
+    __syncthreads();
+    if (upd) {
+      T acc = T(0);
+      const T* pp = part + (rt >> 5) * parts * kSlice + (rt & 31);
+      for (int k = 0; k < parts; ++k)
+        acc += pp[k * kSlice];
+      const T v = xo[urow] + omega * (dr * (br - acc));
+      const uint32_t a = xbase + uint32_t((1 - cur) * np + urow) * uint32_t(sizeof(T));
+      for (uint32_t r = sub; r < ctas; r += share)
+        send_counted<T>(a, mbar, r, v);
+    }
+    // all n values of this sweep (bounded: the wait always ends)
+    const uint32_t phase = (turn >> 1) & 1;
+    const unsigned long long t0 = global_ns();
+    for (;;) {
+      uint32_t done;
+      asm volatile("{\n\t.reg .pred p;\n\t"
+                   "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+                   "selp.u32 %0, 1, 0, p;\n\t}"
+                   : "=r"(done) : "r"(mbar), "r"(phase) : "memory");
+      if (done)
+        break;
+      if (global_ns() - t0 > wait_ns) {
+        atomicExch(err, 1);
+        break;
+      }
+    }
+    cur = 1 - cur;
+  }
+  cluster_barrier(); // nothing is under way to a CTA that has left
+  if (upd && sub == 0)
+    x[urow] = xs[cur * np + urow];
+}
+
 // phantoms: arrivals each grid barrier waits for beyond the grid's own CTAs
 // (0 in every solve; a test sets it to make the bounded wait run out).
 template<class T, int THREADS, bool CLUSTER>

@@ -795,35 +795,34 @@ throw_if_wait_ended(Context& c)
   throw Error{ GB_ETIMEOUT, "a dependency wait of the block ILU gave up waiting" };
 }
 
-// CTAs of the largest cluster the device runs k_ilu_cluster with.
+// CTAs of the largest cluster (16, a size that is not portable, or 8) the
+// device runs the kernel with.
+template<class K>
 static int
-ilu_max_ctas(Context& c)
+max_ctas(K* kern, int threads, size_t smem)
 {
-  if (c.ilu_max_ctas)
-    return c.ilu_max_ctas;
-  int size = 8; // the largest portable cluster
-  auto* kern = k_ilu_cluster<1, double>;
+  int size = 8;
   if (cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) ==
         cudaSuccess &&
-      cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           int(kIluClusterBytes + 32)) == cudaSuccess) {
+      cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)) ==
+        cudaSuccess) {
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(kIluClusterMax);
-    cfg.blockDim = dim3(kIluClusterThreads);
-    cfg.dynamicSmemBytes = kIluClusterBytes + 32;
+    cfg.gridDim = dim3(16);
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = kIluClusterMax;
+    attr[0].val.clusterDim.x = 16;
     attr[0].val.clusterDim.y = 1;
     attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     int n = 0;
     if (cudaOccupancyMaxActiveClusters(&n, kern, &cfg) == cudaSuccess && n > 0)
-      size = kIluClusterMax;
+      size = 16;
   }
   cudaGetLastError(); // a refused query leaves no error behind
-  return c.ilu_max_ctas = size;
+  return size;
 }
 
 // How the level's rows are shared out among the CTAs of k_ilu_cluster, and the
@@ -840,7 +839,9 @@ ilu_groups(Context& c, Level& L, const std::vector<int> (&lev)[2], const int (&n
   const int64_t n = L.n;
   if (!c.ilu_cluster || (n + 1) * L.B >= (int64_t(1) << kIluOwnerShift))
     return;
-  const int most = ilu_max_ctas(c);
+  if (!c.ilu_max_ctas)
+    c.ilu_max_ctas = max_ctas(k_ilu_cluster<1, double>, kIluClusterThreads, kIluClusterBytes + 32);
+  const int most = c.ilu_max_ctas;
   auto bytes = [&](int ctas, size_t size) { return size_t((n + ctas - 1) / ctas) * L.B * size; };
   const size_t size = bytes(most, 8) <= kIluClusterBytes ? 8 : 4;
   if (bytes(most, size) > kIluClusterBytes)
@@ -1243,6 +1244,8 @@ ensure_work(Context& c)
   }
   for (int l = 0; l < c.nlevels; ++l)
     ensure_pf_scratch(c, c.L[l].n);
+  if (c.exact_ctas < 0)
+    c.exact_ctas = max_ctas(k_exact_sweeps<double>, kExactWarps * 32, kExactBytes);
   for (int l = 0; l < c.nlevels; ++l) {
     Level& L = c.L[l];
     if (!L.has_hn())
