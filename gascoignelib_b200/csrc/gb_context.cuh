@@ -798,28 +798,28 @@ spmv(Context& c, const Level& L, const Sell& S, const TX* x, TO* y, const TO* b,
     }
   }
   const SellView<TV> A = view<TV>(S, sell_vals<TV>(S));
-  const int nb = blocks_for(S.n, kSpmvThreads);
+  const int nb = blocks_for(S.n, kRowThreads);
   const uint8_t* dm = L.dirmask.p;
   // FP32 values only: measured on C2, the FP32 cycle gains (1.550 -> 1.544 ms)
   // where the FP64 one, already at 64 registers for its smoother, loses
   const bool small = sizeof(TV) == 4 && S.n < kSpmvSmallRows;
   if (S.pat && small)
-    launch(c, k_spmv<MODE, TV, TX, TO, kColPat, true>, nb, kSpmvThreads, A, x, y, b, dinv,
+    launch(c, k_spmv<MODE, TV, TX, TO, kColPat, true>, nb, kRowThreads, A, x, y, b, dinv,
            dm, alpha, yidx, ystride, xcopy);
   else if (S.pat)
-    launch(c, k_spmv<MODE, TV, TX, TO, kColPat>, nb, kSpmvThreads, A, x, y, b, dinv, dm,
+    launch(c, k_spmv<MODE, TV, TX, TO, kColPat>, nb, kRowThreads, A, x, y, b, dinv, dm,
            alpha, yidx, ystride, xcopy);
   else if (A.c16 && small)
-    launch(c, k_spmv<MODE, TV, TX, TO, kColOff16, true>, nb, kSpmvThreads, A, x, y, b, dinv,
+    launch(c, k_spmv<MODE, TV, TX, TO, kColOff16, true>, nb, kRowThreads, A, x, y, b, dinv,
            dm, alpha, yidx, ystride, xcopy);
   else if (A.c16)
-    launch(c, k_spmv<MODE, TV, TX, TO, kColOff16>, nb, kSpmvThreads, A, x, y, b, dinv, dm,
+    launch(c, k_spmv<MODE, TV, TX, TO, kColOff16>, nb, kRowThreads, A, x, y, b, dinv, dm,
            alpha, yidx, ystride, xcopy);
   else if (small)
-    launch(c, k_spmv<MODE, TV, TX, TO, kColIdx, true>, nb, kSpmvThreads, A, x, y, b, dinv,
+    launch(c, k_spmv<MODE, TV, TX, TO, kColIdx, true>, nb, kRowThreads, A, x, y, b, dinv,
            dm, alpha, yidx, ystride, xcopy);
   else
-    launch(c, k_spmv<MODE, TV, TX, TO, kColIdx>, nb, kSpmvThreads, A, x, y, b, dinv, dm,
+    launch(c, k_spmv<MODE, TV, TX, TO, kColIdx>, nb, kRowThreads, A, x, y, b, dinv, dm,
            alpha, yidx, ystride, xcopy);
 }
 

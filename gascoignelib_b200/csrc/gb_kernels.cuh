@@ -177,8 +177,16 @@ constexpr int spmv_min_blocks()
                                   : (MODE == 0 ? GB_SPMV_MINB_F64AX : GB_SPMV_MINB_F64));
 }
 
+// Threads per CTA. The rows of a length window are sorted, so a CTA's warps
+// have rows of different lengths and hold its registers until the longest is
+// done (Q2: 27 to 125 entries; 67 % of the warps active with CTAs of 8 warps).
+// FP32 sweep with CTAs of 256 / 128 / 64 threads: 40^3 Q2 with a refined ball
+// 23.1 / 20.2 / 20.9 us, 64^3 Q1 11.4 / 10.9 / 12.7 us; FP64, 80^3 Q2 65.0 /
+// 62.0 / 61.7 us.
+constexpr int kRowThreads = 128;
 template<int MODE, class TV, class TX, class TO, int CM, bool SMALL = false>
-__global__ void __launch_bounds__(kSpmvThreads, (spmv_min_blocks<MODE, TV, SMALL>()))
+__global__ void __launch_bounds__(kRowThreads,
+                                  (spmv_min_blocks<MODE, TV, SMALL>() * 256 / kRowThreads))
 k_spmv(SellView<TV> A, const TX* __restrict__ x, TO* __restrict__ y,
        const TO* __restrict__ b, const TV* __restrict__ dinv,
        const uint8_t* __restrict__ dirmask, double alpha_,
@@ -209,11 +217,16 @@ k_spmv(SellView<TV> A, const TX* __restrict__ x, TO* __restrict__ y,
   };
   for (int j0 = 0; j0 < w; j0 += kChunk) {
     TA av[kChunk], xv[kChunk];
+    int4 o4;
 #pragma unroll
     for (int q = 0; q < kChunk; ++q) {
       const int j = j0 + q;
       if (j < w) {
-        const int c = PAT                ? row + ldg(cp + j)
+        // pattern rows are multiples of 16 bytes: four offsets a load (the
+        // load unit is what a row waits for: 80^3 Q2, FP32 47.2 -> 43.1 us)
+        if (PAT && q % 4 == 0)
+          o4 = ldg(reinterpret_cast<const int4*>(cp + j));
+        const int c = PAT ? row + (q % 4 == 0 ? o4.x : q % 4 == 1 ? o4.y : q % 4 == 2 ? o4.z : o4.w)
                       : CM == kColOff16 ? row + int(ldg(hp + j * kSlice))
                                         : ldg(cp + j * kSlice);
         av[q] = static_cast<TA>(ldg(vp + j * kSlice));
