@@ -408,6 +408,7 @@ struct gb_ctx
     int64_t version = -1;
     int setup_k = 0, outer_k = 0, inner_k = 0;
   } fg[2][2]; // [operator transposed][cycle precision]
+  FGraph lg[2]; // the left-preconditioned solver's, [operator transposed]
   // level operators: A (0) or A^T (1) for every solver step (gb_set_operator)
   int transposed = 0;
   // coarse-level kernel: levels 0..coarse_root, programs per entry state
@@ -502,13 +503,17 @@ struct gb_ctx
       cudaEventDestroy(p.e0);
       cudaEventDestroy(p.e1);
     }
+    auto drop = [](FGraph& g) {
+      if (g.exec)
+        cudaGraphExecDestroy(g.exec);
+      if (g.graph)
+        cudaGraphDestroy(g.graph);
+    };
     for (auto& row : fg)
-      for (auto& g : row) {
-        if (g.exec)
-          cudaGraphExecDestroy(g.exec);
-        if (g.graph)
-          cudaGraphDestroy(g.graph);
-      }
+      for (auto& g : row)
+        drop(g);
+    for (auto& g : lg)
+      drop(g);
   }
 };
 

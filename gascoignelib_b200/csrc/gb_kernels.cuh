@@ -933,10 +933,13 @@ cginfo_check(CGInfoDev& I, double resi)
 
 // gamma[0] = rho, inv = 1/rho (GMRES::solve, LinAlg/gmres.cc:182-192)
 static __global__ void
-k_gmres_init(GmresDev* G, const double* rho_p)
+k_gmres_init(GmresDev* G, const double* rho_p, cudaGraphConditionalHandle loop, int use_cond)
 {
   GB_PDL_ENTRY();
   double rho = *rho_p;
+  G->j = 0;
+  if (use_cond)
+    cudaGraphSetConditional(loop, rho == 0.0 ? 0 : 1);
   G->gamma[0] = rho;
   G->zero_rho = (rho == 0.0);
   G->inv = 1.0 / rho;
@@ -1197,7 +1200,8 @@ k_scale_idx(int64_t n, double* __restrict__ V, const int* __restrict__ jp,
     v[i] = s * v[i];
 }
 
-// Classical Gram-Schmidt, twice (CGS2), on w = V_{j+1} against V_0..V_j, j = G->j:
+// Classical Gram-Schmidt, twice (CGS2), on w = V_{j+1} against V_0..V_j, j = G->j
+// (pass 0 reads w from src0 when that is set, and stores it):
 //  MODE 0: c1[i] = <w, V_i>;                         H[j][i]  = c1[i]
 //  MODE 1: w -= sum_i c1[i] V_i; c2[i] = <w, V_i>;   H[j][i] += c2[i]
 //  MODE 2: w -= sum_i c2[i] V_i; s = ||w||;          H[j][j+1] = s
@@ -1218,12 +1222,20 @@ constexpr int kCgsThreads = 256;
 #endif
 constexpr int kCgsMaxBlocks = GB_CGS_MAX_BLOCKS;
 
-static __device__ void fg_step(GmresDev* G, cudaGraphConditionalHandle inner, int m,
-                        int use_cond);
+// What ends a step of the Arnoldi loop: the flexible solver's aim on the true
+// residual, or CGInfo's rule (left-preconditioned, LinAlg/gmres.cc).
+enum StepRule
+{
+  kStepFlexible = 0,
+  kStepCgInfo = 1
+};
+static __device__ void arnoldi_step(GmresDev* G, double* h, double* ci, double* si,
+                                    cudaGraphConditionalHandle inner, int m, int use_cond,
+                                    int rule);
 
 template<int MODE, int NV>
 __device__ __forceinline__ void
-cgs_pass(int64_t n, const double* __restrict__ V, double* __restrict__ w,
+cgs_pass(int64_t n, const double* __restrict__ V, const double* src, double* w,
          const volatile double* coef, double (*s_warp)[kCgsMaxJ + 1])
 {
   // coef (shared memory) is read where it is used: volatile keeps the
@@ -1241,7 +1253,9 @@ cgs_pass(int64_t n, const double* __restrict__ V, double* __restrict__ w,
   double accn = 0.0; // MODE 1: ||w'||^2
   const int64_t stride = int64_t(gridDim.x) * kCgsThreads;
   for (int64_t r = int64_t(blockIdx.x) * kCgsThreads + tid; r < n; r += stride) {
-    double t = w[r];
+    double t = src[r];
+    if (MODE == 0 && src != w)
+      w[r] = t;
     if (MODE >= 1) {
 #pragma unroll
       for (int g = 0; g < NV; g += kGroup) {
@@ -1293,7 +1307,7 @@ cgs_pass(int64_t n, const double* __restrict__ V, double* __restrict__ w,
 }
 
 // MODE 1 also forms the norm of the new basis vector and performs the Givens
-// update and the loop test (fg_step) in its last block: with w' the vector
+// update and the loop test (arnoldi_step) in its last block: with w' the vector
 // after the first pass and c2 the second pass's coefficients, the basis is
 // orthonormal, so ||w''||^2 = ||w'||^2 - ||c2||^2 (c2 is tiny against w' after
 // a first CGS pass, so the difference loses no digits; it is clamped at 0,
@@ -1303,27 +1317,29 @@ cgs_pass(int64_t n, const double* __restrict__ V, double* __restrict__ w,
 // (the update-and-norm pass of the plain CGS2 order) is not launched.
 template<int MODE>
 __global__ void __launch_bounds__(kCgsThreads, 2)
-k_cgs(int64_t n, double* __restrict__ V, GmresDev* G, double* partials,
-      unsigned* ticket, cudaGraphConditionalHandle inner, int m, int use_cond)
+k_cgs(int64_t n, double* __restrict__ V, const double* src0, GmresDev* G, double* partials,
+      unsigned* ticket, cudaGraphConditionalHandle inner, int m, int use_cond, int rule)
 {
   GB_PDL_ENTRY();
   constexpr int kWarps = kCgsThreads / 32;
   __shared__ double s_coef[kCgsMaxJ];
   __shared__ double s_warp[kWarps][kCgsMaxJ + 1];
   __shared__ double s_red[kCgsMaxJ + 1];
+  __shared__ double s_h[kCgsMaxJ + 2], s_ci[kCgsMaxJ + 1], s_si[kCgsMaxJ + 1];
   __shared__ bool am_last;
   const int j = G->j;
   const int nv = j + 1;
   const int nred = (MODE == 2) ? 1 : (MODE == 1 ? nv + 1 : nv);
   const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
   double* w = V + int64_t(j + 1) * n;
+  const double* src = MODE == 0 && src0 ? src0 : w;
   if (MODE >= 1 && tid < kCgsMaxJ)
     s_coef[tid] = (tid < nv) ? (MODE == 1 ? G->d[tid] : G->d2[tid]) : 0.0;
   __syncthreads();
   switch (nv) {
 #define GB_CGS_CASE(K)                                                          \
   case K:                                                                      \
-    cgs_pass<MODE, K>(n, V, w, s_coef, s_warp);                                \
+    cgs_pass<MODE, K>(n, V, src, w, s_coef, s_warp);                                \
     break;
     GB_CGS_CASE(1) GB_CGS_CASE(2) GB_CGS_CASE(3) GB_CGS_CASE(4) GB_CGS_CASE(5)
     GB_CGS_CASE(6) GB_CGS_CASE(7) GB_CGS_CASE(8) GB_CGS_CASE(9) GB_CGS_CASE(10)
@@ -1361,76 +1377,90 @@ k_cgs(int64_t n, double* __restrict__ V, GmresDev* G, double* partials,
       s_red[i] = v;
   }
   __syncthreads();
-  if (tid == 0) {
-    if (MODE == 0) {
-      for (int i = 0; i < nv; ++i) {
-        G->d[i] = s_red[i];
-        G->H[j][i] = s_red[i];
-      }
-    } else if (MODE == 1) {
-      double c2 = 0.0;
-      for (int i = 0; i < nv; ++i) {
-        G->d2[i] = s_red[i];
-        G->H[j][i] += s_red[i];
-        c2 = fma(s_red[i], s_red[i], c2);
-      }
-      const double sv = sqrt(fmax(s_red[nv] - c2, 0.0));
-      G->H[j][j + 1] = sv;
-      G->s = sv;
-    } else {
-      const double sv = sqrt(s_red[0]);
-      G->H[j][j + 1] = sv;
-      G->s = sv;
+  // one thread per coefficient; only the rotations, a recurrence, run on one
+  // thread, on copies in shared memory
+  if (MODE == 0) {
+    if (tid < nv) {
+      G->d[tid] = s_red[tid];
+      G->H[j][tid] = s_red[tid];
     }
-    *ticket = 0u;
-    if (MODE >= 1) {
-      __threadfence_block();
-      fg_step(G, inner, m, use_cond);
-    }
+    if (tid == 0)
+      *ticket = 0u;
+    return;
   }
+  if (MODE == 1 && tid < nv) {
+    G->d2[tid] = s_red[tid];
+    s_h[tid] = G->H[j][tid] + s_red[tid];
+  }
+  if (tid < j) {
+    s_ci[tid] = G->ci[tid];
+    s_si[tid] = G->si[tid];
+  }
+  __syncthreads();
+  if (tid == 0) {
+    double sv;
+    if (MODE == 1) {
+      double c2 = 0.0;
+      for (int i = 0; i < nv; ++i)
+        c2 = fma(s_red[i], s_red[i], c2);
+      sv = sqrt(fmax(s_red[nv] - c2, 0.0));
+    } else {
+      sv = sqrt(s_red[0]);
+      for (int i = 0; i < nv; ++i)
+        s_h[i] = G->H[j][i];
+    }
+    s_h[nv] = sv;
+    G->s = sv;
+    *ticket = 0u;
+    arnoldi_step(G, s_h, s_ci, s_si, inner, m, use_cond, rule);
+  }
+  __syncthreads();
+  if (tid <= nv)
+    G->H[j][tid] = s_h[tid];
 }
 
 // Givens update of column j (LinAlg/gmres.cc:88-104 applied to the flexible
-// Hessenberg), residual estimate |gamma[j+1]| = ||b - A x_j|| in exact
-// arithmetic, then j += 1 and the inner loop condition.
+// Hessenberg; h, ci, si in shared memory), residual estimate |gamma[j+1]| =
+// ||b - A x_j|| in exact arithmetic (left: of the preconditioned system), then
+// j += 1 and the loop condition.
 static __device__ void
-fg_step(GmresDev* G, cudaGraphConditionalHandle inner, int m, int use_cond)
+arnoldi_step(GmresDev* G, double* h, double* ci, double* si, cudaGraphConditionalHandle inner,
+             int m, int use_cond, int rule)
 {
   const int last = G->j, dim = last + 1;
-  double* h = G->H[last];
   const double s = h[dim];
   G->inv = 1.0 / s;
   for (int i = 0; i < last; i++) {
     double dummy = h[i];
-    h[i] = G->ci[i] * dummy + G->si[i] * h[i + 1];
-    h[i + 1] = -G->si[i] * dummy + G->ci[i] * h[i + 1];
+    h[i] = ci[i] * dummy + si[i] * h[i + 1];
+    h[i + 1] = -si[i] * dummy + ci[i] * h[i + 1];
   }
   double r = 1. / sqrt(h[last] * h[last] + h[last + 1] * h[last + 1]);
-  G->si[last] = h[last + 1] * r;
-  G->ci[last] = h[last] * r;
-  h[last] = G->ci[last] * h[last] + G->si[last] * h[last + 1];
-  G->gamma[last + 1] = -G->si[last] * G->gamma[last];
-  G->gamma[last] *= G->ci[last];
-  const double rho = fabs(G->gamma[dim]);
-  if (G->total < kMaxV)
-    G->hist[G->total] = rho;
-  G->info.residual = rho;
-  G->info.iteration += 1;
-  G->total += 1;
+  const double sl = h[last + 1] * r, cl = h[last] * r;
+  G->si[last] = sl;
+  G->ci[last] = cl;
+  h[last] = cl * h[last] + sl * h[last + 1];
+  const double gl = G->gamma[last], gd = -sl * gl;
+  G->gamma[dim] = gd;
+  G->gamma[last] = gl * cl;
+  const double rho = fabs(gd);
   G->j = dim;
-  const double aim = fmax(G->info.tol * G->bnorm, G->info.globaltol);
-  const int reached = (rho <= aim) || dim >= m || G->total >= G->info.maxiter ||
-                      !(rho == rho);
+  int reached;
+  if (rule == kStepCgInfo) {
+    G->hist[last] = rho;
+    reached = cginfo_check(G->info, rho) || dim >= m;
+  } else {
+    if (G->total < kMaxV)
+      G->hist[G->total] = rho;
+    G->info.residual = rho;
+    G->info.iteration += 1;
+    G->total += 1;
+    const double aim = fmax(G->info.tol * G->bnorm, G->info.globaltol);
+    reached = (rho <= aim) || dim >= m || G->total >= G->info.maxiter || !(rho == rho);
+  }
   G->reached = reached;
   if (use_cond)
     cudaGraphSetConditional(inner, reached ? 0 : 1);
-}
-
-static __global__ void
-k_fg_step(GmresDev* G, cudaGraphConditionalHandle inner, int m, int use_cond)
-{
-  GB_PDL_ENTRY();
-  fg_step(G, inner, m, use_cond);
 }
 
 // hs = H^-1 gamma on the first G->j columns (Common/mult.h:130-141)
