@@ -651,7 +651,7 @@ gb_level_set_pfilter(gb_ctx* ctx, int lvl, int comp_mask, const double* weights,
     GB_CUDA(h2d(ctx->stream, L.pf_w.p, weights, L.n * sizeof(double)));
   }
   if (comp_mask)
-    ensure_pf_scratch(*ctx, L.n);
+    ensure_pf_scratch(*ctx, L);
   L.pf_mask = comp_mask;
   L.pf_domain = domain;
   L.nhanging = nhanging;
@@ -915,15 +915,15 @@ gb_restrict_zero(gb_ctx* ctx, int lvl, int coarse_id, int fine_id)
                (const double*)nullptr, (double*)nullptr, 0.0);
       break;
     case 2:
-      launch(*ctx, k_restrict_b<double, 2>, nb, 256, T.nc, tp, te, f, cc, nm, -1,
+      launch(*ctx, k_restrict_b<double, 2>, blocks_for(int64_t(T.nc) * 2, 256), 256, T.nc, tp, te, f, cc, nm, -1,
              (const double*)nullptr);
       break;
     case 3:
-      launch(*ctx, k_restrict_b<double, 3>, nb, 256, T.nc, tp, te, f, cc, nm, -1,
+      launch(*ctx, k_restrict_b<double, 3>, blocks_for(int64_t(T.nc) * 3, 256), 256, T.nc, tp, te, f, cc, nm, -1,
              (const double*)nullptr);
       break;
     default:
-      launch(*ctx, k_restrict_b<double, 4>, nb, 256, T.nc, tp, te, f, cc, nm, -1,
+      launch(*ctx, k_restrict_b<double, 4>, blocks_for(int64_t(T.nc) * 4, 256), 256, T.nc, tp, te, f, cc, nm, -1,
              (const double*)nullptr);
   }
   GB_API_END
@@ -947,13 +947,13 @@ gb_prolongate_add(gb_ctx* ctx, int lvl, int fine_id, int coarse_id)
       launch(*ctx, k_prolong<0, double>, nb, 256, T.nf, tp, te, cc, f, nm, 1.0);
       break;
     case 2:
-      launch(*ctx, k_prolong_b<0, double, 2>, nb, 256, T.nf, tp, te, cc, f, nm, 1.0);
+      launch(*ctx, k_prolong_b<0, double, 2>, blocks_for(int64_t(T.nf) * 2, 256), 256, T.nf, tp, te, cc, f, nm, 1.0);
       break;
     case 3:
-      launch(*ctx, k_prolong_b<0, double, 3>, nb, 256, T.nf, tp, te, cc, f, nm, 1.0);
+      launch(*ctx, k_prolong_b<0, double, 3>, blocks_for(int64_t(T.nf) * 3, 256), 256, T.nf, tp, te, cc, f, nm, 1.0);
       break;
     default:
-      launch(*ctx, k_prolong_b<0, double, 4>, nb, 256, T.nf, tp, te, cc, f, nm, 1.0);
+      launch(*ctx, k_prolong_b<0, double, 4>, blocks_for(int64_t(T.nf) * 4, 256), 256, T.nf, tp, te, cc, f, nm, 1.0);
   }
   GB_API_END
 }

@@ -90,6 +90,85 @@ k_bspmv(SellView<TV> A, const TX* __restrict__ x, TO* __restrict__ y,
   }
 }
 
+// Component r of a block row: its part of every block's product, in the order
+// of k_bspmv (a row's sums over the block, then added), so the same bits.
+template<int B, bool NEG, bool PAT, class TV, class TX, class TA>
+__device__ __forceinline__ TA
+bspmv_component(const SellView<TV>& A, const TX* __restrict__ x, int s, int lane, int row, int r,
+                TA acc)
+{
+  constexpr int B2 = B * B;
+  const int beg = A.sptr[s];
+  const int w = (A.sptr[s + 1] - beg) >> 5;
+  const TV* vp = A.val + int64_t(beg) * B2 + r * B * kSlice + lane;
+  const int* cp = PAT ? (A.ptab + int(A.pid[row]) * A.W) : (A.col + beg + lane);
+  constexpr int U = 4; // blocks in flight
+  for (int j0 = 0; j0 < w; j0 += U) {
+    TA xv[U][B], m[U][B];
+#pragma unroll
+    for (int q = 0; q < U; ++q) {
+      const int j = j0 + q;
+      const int c = j >= w ? row : PAT ? row + ldg(cp + j) : ldg(cp + j * kSlice);
+#pragma unroll
+      for (int k = 0; k < B; ++k) {
+        xv[q][k] = j < w ? static_cast<TA>(ldg(x + int64_t(c) * B + k)) : TA(0);
+        m[q][k] = j < w ? static_cast<TA>(ldg(vp + (int64_t(j) * B2 + k) * kSlice)) : TA(0);
+      }
+    }
+#pragma unroll
+    for (int q = 0; q < U; ++q) {
+      TA sum = TA(0);
+#pragma unroll
+      for (int k = 0; k < B; ++k)
+        sum = fma(m[q][k], xv[q][k], sum);
+      acc = NEG ? acc - sum : acc + sum; // past the end: a sum of 0
+    }
+  }
+  return acc;
+}
+
+// k_bspmv with a thread per row and component (warp = slice and component): a
+// thread has B of a block's B^2 values to load, and there are B times as many
+// threads. For the levels of at most kBlockSplitRows rows, whose one thread per
+// row leaves most of the GPU idle and is a chain of 27 x B^2 loads. Measured
+// with events around the launch: residual of 17^3 rows, B = 4, FP64 30 -> 15
+// us; of the seven levels below 513^2 rows, B = 3, FP32 about 14 -> 11.8 us
+// each. On the 513^2 level itself the x loads, B times as many, cost more than
+// they gain (the solve 13.9 -> 14.3 ms), so it keeps one thread per row.
+constexpr int64_t kBlockSplitRows = 100000;
+template<int MODE, int B, class TV, class TX, class TO, bool PAT>
+__global__ void __launch_bounds__(kSpmvThreads, 2)
+k_bspmv_split(SellView<TV> A, const TX* __restrict__ x, TO* __restrict__ y,
+              const TO* __restrict__ b, const uint8_t* __restrict__ dirmask, double alpha_,
+              const int* __restrict__ yidx, int64_t ystride, TX* __restrict__ xcopy)
+{
+  GB_PDL_ENTRY();
+  using TA = typename Acc<TV, TO>::type;
+  constexpr bool NEG = MODE == kResid || MODE == kResidDir;
+  const int wid = (blockIdx.x * kSpmvThreads + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+  const int s = wid / B, r = wid % B, slot = s * kSlice + lane;
+  if (slot >= A.n)
+    return;
+  const int row = A.perm ? __ldg(A.perm + slot) : slot;
+  const int64_t o = int64_t(row) * B + r;
+  const TA acc = bspmv_component<B, NEG, PAT, TV, TX, TA>(
+    A, x, s, lane, row, r, NEG ? static_cast<TA>(b[o]) : TA(0));
+  const TA alpha = static_cast<TA>(alpha_);
+  if (yidx) {
+    const int64_t jj = *yidx;
+    xcopy[jj * ystride + o] = x[o];
+    y += (jj + 1) * ystride;
+  }
+  if (MODE == kAx)
+    y[o] = static_cast<TO>(alpha * acc);
+  else if (MODE == kAddAx)
+    y[o] = static_cast<TO>(static_cast<TA>(y[o]) + alpha * acc);
+  else if (MODE == kResid)
+    y[o] = static_cast<TO>(acc);
+  else
+    y[o] = dirmask[o] ? TO(0) : static_cast<TO>(acc);
+}
+
 // y = b - A x on block rows with the pressure filter's plain mean of
 // component pc of y (StdSolver::MatrixResidual with SubtractMeanAlgebraic):
 // the last block writes sum / denom to *mean; consumers subtract it on read.
@@ -142,6 +221,32 @@ k_bspmv_resid_mean(SellView<TV> A, const T* __restrict__ x, T* __restrict__ y,
       if (r == pc)
         v = static_cast<double>(o);
     }
+  }
+  v = block_sum(v, sh);
+  red_finish(partials, ticket, v, RedOut{ mean, nullptr, nullptr, 0, denom }, sh);
+}
+
+// The same with a thread per row and component (k_bspmv_split's rule).
+template<int B, class TV, class T, bool PAT>
+__global__ void __launch_bounds__(kSpmvThreads, 2)
+k_bspmv_resid_mean_split(SellView<TV> A, const T* __restrict__ x, T* __restrict__ y,
+                         const T* __restrict__ b, int pc, double denom, double* partials,
+                         unsigned* ticket, double* mean)
+{
+  GB_PDL_ENTRY();
+  using TA = typename Acc<TV, T>::type;
+  __shared__ double sh[32];
+  const int wid = (blockIdx.x * kSpmvThreads + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+  const int s = wid / B, r = wid % B, slot = s * kSlice + lane;
+  double v = 0.0;
+  if (slot < A.n) {
+    const int row = A.perm ? __ldg(A.perm + slot) : slot;
+    const int64_t o = int64_t(row) * B + r;
+    const T res = static_cast<T>(bspmv_component<B, true, PAT, TV, T, TA>(
+      A, x, s, lane, row, r, static_cast<TA>(b[o])));
+    y[o] = res;
+    if (r == pc)
+      v = static_cast<double>(res);
   }
   v = block_sum(v, sh);
   red_finish(partials, ticket, v, RedOut{ mean, nullptr, nullptr, 0, denom }, sh);
@@ -221,82 +326,82 @@ k_block_jacobi_apply(int n, const TV* __restrict__ dinv, const T* __restrict__ h
   }
 }
 
-// Block transfers: the scalar tables applied to each of the B components.
-// acc holds the starting values (0, or the target for an in-place add: the
-// weights are powers of two, so each fused add rounds like the reference's
-// y += w x).
+// Block transfers: the scalar tables applied to each of the B components, one
+// thread per node and component (the B threads of a node read B consecutive
+// values), eight entries in flight. The sum runs over the entries in order from
+// acc (0, or the target for an in-place add: the weights are powers of two, so
+// each fused add rounds like the reference's y += w x). Component pc is read
+// minus smean.
 template<class T, int B>
-__device__ __forceinline__ void
-transfer_row_b(const int* __restrict__ tsp, const uint32_t* __restrict__ tent,
-               const T* __restrict__ src, int i, T (&acc)[B], int pc = -1,
-               double smean = 0.0)
+__device__ __forceinline__ T
+transfer_dof(const int* __restrict__ tsp, const uint32_t* __restrict__ tent,
+             const T* __restrict__ src, int i, int c, T acc, bool sub = false,
+             double smean = 0.0)
 {
   const int beg = __ldg(tsp + (i >> 5));
   const int w = (__ldg(tsp + (i >> 5) + 1) - beg) >> 5;
   const uint32_t* ep = tent + beg + (i & 31);
-  for (int j = 0; j < w; ++j) {
-    const uint32_t e = __ldg(ep + j * kSlice);
-    const T wgt = wcode<T>(e);
-    const T* sp = src + int64_t(e & kIdxMask) * B;
+  for (int j0 = 0; j0 < w; j0 += 8) {
+    const uint32_t* pe[8];
 #pragma unroll
-    for (int c = 0; c < B; ++c) {
-      const T sv = c == pc ? static_cast<T>(static_cast<double>(__ldg(sp + c)) - smean)
-                           : __ldg(sp + c);
-      acc[c] = fma(wgt, sv, acc[c]);
-    }
+    for (int q = 0; q < 8; ++q)
+      pe[q] = ep + min(j0 + q, w - 1) * kSlice;
+    uint32_t e[8];
+    ld8(e, pe);
+    const T* ps[8];
+#pragma unroll
+    for (int q = 0; q < 8; ++q)
+      ps[q] = src + int64_t(e[q] & kIdxMask) * B + c;
+    T f[8];
+    ld8(f, ps);
+#pragma unroll
+    for (int q = 0; q < 8; ++q)
+      if (j0 + q < w) {
+        const T sv = sub ? static_cast<T>(static_cast<double>(f[q]) - smean) : f[q];
+        acc = fma(wcode<T>(e[q]), sv, acc);
+      }
   }
+  return acc;
 }
 
 // fine's component pc is read minus *smean when smean is set (the filtered
 // residual of MatrixResidual, restricted).
 template<class T, int B>
-__global__ void
+__global__ void __launch_bounds__(256)
 k_restrict_b(int nc, const int* __restrict__ tsp, const uint32_t* __restrict__ tent,
              const T* __restrict__ fine, T* __restrict__ coarse,
              const uint8_t* __restrict__ cdir, int pc = -1,
              const double* __restrict__ smean = nullptr)
 {
   GB_PDL_ENTRY();
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  const int64_t d = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
+  const int i = static_cast<int>(d / B), c = static_cast<int>(d % B);
   if (i >= nc)
     return;
-  T acc[B];
-#pragma unroll
-  for (int c = 0; c < B; ++c)
-    acc[c] = T(0);
-  transfer_row_b<T, B>(tsp, tent, fine, i, acc, smean ? pc : -1, smean ? *smean : 0.0);
-#pragma unroll
-  for (int c = 0; c < B; ++c) {
-    const int64_t d = int64_t(i) * B + c;
-    coarse[d] = (cdir && cdir[d]) ? T(0) : acc[c];
-  }
+  const T acc = transfer_dof<T, B>(tsp, tent, fine, i, c, T(0), smean && c == pc,
+                                   smean ? *smean : 0.0);
+  coarse[d] = (cdir && cdir[d]) ? T(0) : acc;
 }
 
 template<int MODE, class T, int B>
-__global__ void
+__global__ void __launch_bounds__(256)
 k_prolong_b(int nf, const int* __restrict__ tsp, const uint32_t* __restrict__ tent,
             const T* __restrict__ coarse, T* __restrict__ fine,
             const uint8_t* __restrict__ fdir, double mgomega)
 {
   GB_PDL_ENTRY();
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  const int64_t d = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
+  const int i = static_cast<int>(d / B), c = static_cast<int>(d % B);
   if (i >= nf)
     return;
-  T acc[B];
-#pragma unroll
-  for (int c = 0; c < B; ++c)
-    acc[c] = MODE == 0 ? fine[int64_t(i) * B + c] : T(0);
-  transfer_row_b<T, B>(tsp, tent, coarse, i, acc);
-#pragma unroll
-  for (int c = 0; c < B; ++c) {
-    const int64_t d = int64_t(i) * B + c;
-    if (MODE == 0) {
-      fine[d] = acc[c];
-    } else {
-      const T a = (fdir && fdir[d]) ? T(0) : acc[c];
-      fine[d] = fine[d] + static_cast<T>(mgomega) * a;
-    }
+  if (MODE == 0) {
+    fine[d] = transfer_dof<T, B>(tsp, tent, coarse, i, c, fine[d]);
+    return;
   }
+  T a = transfer_dof<T, B>(tsp, tent, coarse, i, c, T(0));
+  if (fdir && fdir[d])
+    a = T(0);
+  fine[d] = fine[d] + static_cast<T>(mgomega) * a;
 }
 
 // ------------------------------------------------------ pressure filter
@@ -451,6 +556,60 @@ k_vanka_factor(int npatch, int npp, int B, int M, const int* __restrict__ map,
   }
 }
 
+// Patches of more than 32 unknowns (3D: 108): one CTA of kVankaWide warps per
+// patch, warp q taking the columns j = q, q + kVankaWide, ..; a row's partial
+// sums are added in the warps' order. With a warp per patch the 512 patches of
+// a 17^3 Stokes level were 3.5 warps per SM with 12 loads each in flight: 29 us
+// against 7.4 us for their 48 MB at the copy rate.
+constexpr int kVankaWide = 8;
+template<int R, class TL, class T>
+__global__ void __launch_bounds__(32 * kVankaWide)
+k_vanka_inv_wide(int npatch, int M, int B, const int* __restrict__ pn,
+                 const TL* __restrict__ inv, const T* __restrict__ h, int pc,
+                 const double* __restrict__ hmean, T* __restrict__ hout)
+{
+  GB_PDL_ENTRY();
+  using TA = typename Acc<TL, T>::type;
+  __shared__ TA H[kVankaMaxM];
+  __shared__ TA part[kVankaWide][R * 32];
+  const int wid = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int p = blockIdx.x;
+  const int64_t np = npatch;
+  const double hm = hmean ? *hmean : 0.0;
+  for (int i = threadIdx.x; i < M; i += 32 * kVankaWide) {
+    const int r = i / B, c = i - r * B;
+    const int node = __ldg(pn + r * np + p);
+    const T hv = __ldg(h + int64_t(node) * B + c);
+    H[i] = (hmean && c == pc) ? static_cast<TA>(static_cast<double>(hv) - hm)
+                              : static_cast<TA>(hv);
+  }
+  __syncthreads();
+  const TL* ip = inv + int64_t(p) * M * M + lane;
+  TA acc[R];
+#pragma unroll
+  for (int k = 0; k < R; ++k)
+    acc[k] = TA(0);
+#pragma unroll 7
+  for (int j = wid; j < M; j += kVankaWide) {
+    const TA hj = H[j];
+#pragma unroll
+    for (int k = 0; k < R; ++k)
+      if (lane + 32 * k < M)
+        acc[k] = fma(static_cast<TA>(__ldg(ip + j * M + 32 * k)), hj, acc[k]);
+  }
+#pragma unroll
+  for (int k = 0; k < R; ++k)
+    part[wid][k * 32 + lane] = acc[k];
+  __syncthreads();
+  for (int i = threadIdx.x; i < M; i += 32 * kVankaWide) {
+    TA v = part[0][i];
+#pragma unroll
+    for (int q = 1; q < kVankaWide; ++q)
+      v += part[q][i];
+    hout[int64_t(p) * M + i] = static_cast<T>(v);
+  }
+}
+
 template<int R, class TL, class T>
 __global__ void __launch_bounds__(32 * kVankaWarps)
 k_vanka_inv(int npatch, int M, int B, const int* __restrict__ pn,
@@ -534,9 +693,9 @@ k_vanka_inv_ct(int npatch, int B, const int* __restrict__ pn, const TL* __restri
 }
 
 // u(i, c) = (u_zero ? 0 : u(i, c)) + omega * ((sum over the node's patches of
-// their solution at (i, c)) * (1 / count)). ent packs (patch, local node):
-// patch * 32 + r (npp <= 27). Solution (patch p, local dof q) at
-// hout[q * s1 + p * s2].
+// their solution at (i, c)) * (1 / count)), a thread per node and component.
+// ent packs (patch, local node): patch * 32 + r (npp <= 27). Solution (patch p,
+// local dof q) at hout[p * M + q].
 template<int B, class T>
 __global__ void __launch_bounds__(256)
 k_vanka_gather(int n, const int* __restrict__ nptr, const int* __restrict__ ent,
@@ -546,31 +705,34 @@ k_vanka_gather(int n, const int* __restrict__ nptr, const int* __restrict__ ent,
   GB_PDL_ENTRY();
   using TA = typename Acc<T, T>::type;
   __shared__ double sh[32];
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  const int64_t d = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
+  const int i = static_cast<int>(d / B), c = static_cast<int>(d % B);
   double wv = 0.0;
   if (i < n) {
     const int k0 = __ldg(nptr + i), k1 = __ldg(nptr + i + 1);
-    TA acc[B];
+    TA acc = TA(0);
+    for (int k = k0; k < k1; k += 4) { // four patches' values in flight
+      int e[4];
 #pragma unroll
-    for (int c = 0; c < B; ++c)
-      acc[c] = TA(0);
-    for (int k = k0; k < k1; ++k) {
-      const int e = __ldg(ent + k);
-      const int64_t p = e >> 5, r = e & 31;
+      for (int q = 0; q < 4; ++q)
+        e[q] = k + q < k1 ? __ldg(ent + k + q) : -1;
+      TA v[4];
 #pragma unroll
-      for (int c = 0; c < B; ++c)
-        acc[c] += static_cast<TA>(hout[p * M + r * B + c]);
+      for (int q = 0; q < 4; ++q)
+        v[q] = e[q] >= 0
+                 ? static_cast<TA>(hout[int64_t(e[q] >> 5) * M + (e[q] & 31) * B + c])
+                 : TA(0);
+#pragma unroll
+      for (int q = 0; q < 4; ++q)
+        if (e[q] >= 0)
+          acc += v[q];
     }
     const TA sc = TA(1) / static_cast<TA>(k1 - k0);
-#pragma unroll
-    for (int c = 0; c < B; ++c) {
-      const int64_t d = int64_t(i) * B + c;
-      const TA base = u_zero ? TA(0) : static_cast<TA>(u[d]);
-      const T un = static_cast<T>(base + static_cast<TA>(omega) * (acc[c] * sc));
-      u[d] = un;
-      if (pf.w && c == pf.pc)
-        wv = static_cast<double>(un) * pf.w[i];
-    }
+    const TA base = u_zero ? TA(0) : static_cast<TA>(u[d]);
+    const T un = static_cast<T>(base + static_cast<TA>(omega) * (acc * sc));
+    u[d] = un;
+    if (pf.w && c == pf.pc)
+      wv = static_cast<double>(un) * pf.w[i];
   }
   if (pf.w) {
     wv = block_sum(wv, sh);

@@ -737,7 +737,7 @@ void rows_refresh(Context& c, const Sell& S, bool columns);
 void build_rows(Context& c, Sell& S, const int64_t* rowptr);
 void host_values(Context& c, Level& L);
 void ensure_AT(Context& c, Level& L);
-void ensure_pf_scratch(Context& c, int64_t n);
+void ensure_pf_scratch(Context& c, const Level& L);
 bool direct_on(const Context& c);
 void ensure_vanka(Context& c, Level& L);
 void ensure_ilu(Context& c, Level& L);
@@ -758,6 +758,16 @@ bspmv(Context& c, const Level& L, const Sell& S, const TX* x, TO* y, const TO* b
       const TV* dinv, double alpha, const int* yidx, int64_t ystride, TX* xcopy)
 {
   const SellView<TV> A = view<TV>(S, sell_vals<TV>(S));
+  if constexpr (MODE != kJacobi) { // that mode needs a row's components together
+    if (S.n <= kBlockSplitRows) {
+      const int nb = blocks_for(int64_t(S.nslices) * B * kSlice, kSpmvThreads);
+      launch(c, S.pat ? k_bspmv_split<MODE, B, TV, TX, TO, true>
+                      : k_bspmv_split<MODE, B, TV, TX, TO, false>,
+             nb, kSpmvThreads, A, x, y, b, (const uint8_t*)L.dirmask.p, alpha, yidx, ystride,
+             xcopy);
+      return;
+    }
+  }
   if (S.pat)
     launch(c, k_bspmv<MODE, B, TV, TX, TO, true>, blocks_for(S.n, kSpmvThreads),
            kSpmvThreads, A, x, y, b, dinv, (const uint8_t*)L.dirmask.p, alpha, yidx,

@@ -76,19 +76,19 @@ void Emit<T>::vanka(int l, const T* h, T* u, bool u_zero, const double* hmean)
              (const int*)L.vk_pn.p, inv, h, pc, hmean, out);
       break;
     case 2:
-      launch(c, k_vanka_inv<2, T, T>, nbp, 32 * kVankaWarps, L.npatch, L.vk_M, L.B,
+      launch(c, k_vanka_inv_wide<2, T, T>, L.npatch, 32 * kVankaWide, L.npatch, L.vk_M, L.B,
              (const int*)L.vk_pn.p, inv, h, pc, hmean, out);
       break;
     case 3:
-      launch(c, k_vanka_inv<3, T, T>, nbp, 32 * kVankaWarps, L.npatch, L.vk_M, L.B,
+      launch(c, k_vanka_inv_wide<3, T, T>, L.npatch, 32 * kVankaWide, L.npatch, L.vk_M, L.B,
              (const int*)L.vk_pn.p, inv, h, pc, hmean, out);
       break;
     default:
-      launch(c, k_vanka_inv<4, T, T>, nbp, 32 * kVankaWarps, L.npatch, L.vk_M, L.B,
+      launch(c, k_vanka_inv_wide<4, T, T>, L.npatch, 32 * kVankaWide, L.npatch, L.vk_M, L.B,
              (const int*)L.vk_pn.p, inv, h, pc, hmean, out);
   }
   const PfArgs pf = weighted_mean_args(L);
-  const int nb = blocks_for(L.n, 256);
+  const int nb = blocks_for(L.ndof(), 256);
   switch (L.B) {
     case 1:
       launch(c, k_vanka_gather<1, T>, nb, 256, (int)L.n, (const int*)L.vk_nptr.p,
@@ -123,7 +123,7 @@ int Emit<T>::pf_comp(const Level& L)
 template<class T>
 void Emit<T>::check_pf_scratch(const Level& L) const
 {
-  GB_REQUIRE(c.pfpart.p && c.pfpart.n >= static_cast<size_t>((L.n + 255) / 256 + 1) &&
+  GB_REQUIRE(c.pfpart.p && c.pfpart.n >= static_cast<size_t>((L.ndof() + kSlice * L.B + 255) / 256 + 1) &&
                c.pfticket.p,
              GB_ESTATE, "filter scratch not allocated for this level");
 }
@@ -155,10 +155,12 @@ const double* Emit<T>::resid_mean(int l, const T* u, T* out, const T* b)
   if (L.B > 1) {
     check_pf_scratch(L);
     const SellView<T> A = view<T>(S, sell_vals<T>(S));
-    const int nb = blocks_for(S.n, kSpmvThreads);
+    const bool split = S.n <= kBlockSplitRows;
+    const int nb = split ? blocks_for(int64_t(S.nslices) * S.B * kSlice, kSpmvThreads)
+                         : blocks_for(S.n, kSpmvThreads);
 #define GB_RM(BB, PP)                                                                 \
-launch(c, k_bspmv_resid_mean<BB, T, T, PP>, nb, kSpmvThreads, A, u, out, b, pc, denom, \
-       c.pfpart.p, c.pfticket.p, c.scal.p + 8)
+launch(c, split ? k_bspmv_resid_mean_split<BB, T, T, PP> : k_bspmv_resid_mean<BB, T, T, PP>, \
+       nb, kSpmvThreads, A, u, out, b, pc, denom, c.pfpart.p, c.pfticket.p, c.scal.p + 8)
     if (L.B == 2) {
       if (S.pat) GB_RM(2, true); else GB_RM(2, false);
     } else if (L.B == 3) {
@@ -434,15 +436,15 @@ void Emit<T>::restrict_to(int l, const T* fine, T* coarse, const double* smean, 
       break;
     case 2:
       GB_REQUIRE(!u1, GB_EINVAL, "fused first sweep on a block level");
-      launch(c, k_restrict_b<T, 2>, nb, 256, Tr.nc, Tr.rptr.p, Tr.rent.p, fine, coarse, cm,
+      launch(c, k_restrict_b<T, 2>, blocks_for(int64_t(Tr.nc) * 2, 256), 256, Tr.nc, Tr.rptr.p, Tr.rent.p, fine, coarse, cm,
              pf_comp(c.L[l + 1]), smean);
       break;
     case 3:
-      launch(c, k_restrict_b<T, 3>, nb, 256, Tr.nc, Tr.rptr.p, Tr.rent.p, fine, coarse, cm,
+      launch(c, k_restrict_b<T, 3>, blocks_for(int64_t(Tr.nc) * 3, 256), 256, Tr.nc, Tr.rptr.p, Tr.rent.p, fine, coarse, cm,
              pf_comp(c.L[l + 1]), smean);
       break;
     default:
-      launch(c, k_restrict_b<T, 4>, nb, 256, Tr.nc, Tr.rptr.p, Tr.rent.p, fine, coarse, cm,
+      launch(c, k_restrict_b<T, 4>, blocks_for(int64_t(Tr.nc) * 4, 256), 256, Tr.nc, Tr.rptr.p, Tr.rent.p, fine, coarse, cm,
              pf_comp(c.L[l + 1]), smean);
   }
 }
@@ -505,15 +507,15 @@ void Emit<T>::prolong(int l, const T* coarse, T* fine)
       launch(c, k_prolong<1, T>, nb, 256, Tr.nf, Tr.pptr.p, Tr.pent.p, coarse, fine, fm, mw);
       break;
     case 2:
-      launch(c, k_prolong_b<1, T, 2>, nb, 256, Tr.nf, Tr.pptr.p, Tr.pent.p, coarse, fine,
+      launch(c, k_prolong_b<1, T, 2>, blocks_for(int64_t(Tr.nf) * 2, 256), 256, Tr.nf, Tr.pptr.p, Tr.pent.p, coarse, fine,
              fm, mw);
       break;
     case 3:
-      launch(c, k_prolong_b<1, T, 3>, nb, 256, Tr.nf, Tr.pptr.p, Tr.pent.p, coarse, fine,
+      launch(c, k_prolong_b<1, T, 3>, blocks_for(int64_t(Tr.nf) * 3, 256), 256, Tr.nf, Tr.pptr.p, Tr.pent.p, coarse, fine,
              fm, mw);
       break;
     default:
-      launch(c, k_prolong_b<1, T, 4>, nb, 256, Tr.nf, Tr.pptr.p, Tr.pent.p, coarse, fine,
+      launch(c, k_prolong_b<1, T, 4>, blocks_for(int64_t(Tr.nf) * 4, 256), 256, Tr.nf, Tr.pptr.p, Tr.pent.p, coarse, fine,
              fm, mw);
   }
 }

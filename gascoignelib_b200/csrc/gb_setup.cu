@@ -380,9 +380,10 @@ ensure_AT(Context& c, Level& L)
 // Per-block sums of the filter reductions fused into the residual and update
 // kernels (grid of blocks_for(n, 256) blocks on a level of n nodes).
 void
-ensure_pf_scratch(Context& c, int64_t n)
+ensure_pf_scratch(Context& c, const Level& L)
 {
-  const size_t need = static_cast<size_t>((n + 255) / 256 + 1);
+  // a partial sum per CTA of the kernels with a thread per row and component
+  const size_t need = static_cast<size_t>((L.ndof() + kSlice * L.B + 255) / 256 + 1);
   if (c.pfpart.n < need)
     GB_CUDA(c.pfpart.alloc(need));
   if (c.pfticket.n < 1) {
@@ -1243,7 +1244,7 @@ ensure_work(Context& c)
       ensure_ilu(c, c.L[l]);
   }
   for (int l = 0; l < c.nlevels; ++l)
-    ensure_pf_scratch(c, c.L[l].n);
+    ensure_pf_scratch(c, c.L[l]);
   if (c.exact_ctas < 0)
     c.exact_ctas = max_ctas(k_exact_sweeps<double>, kExactWarps * 32, kExactBytes);
   for (int l = 0; l < c.nlevels; ++l) {
