@@ -144,6 +144,7 @@ struct Sell
   // pattern-compressed form: row r's columns are r + ptab[pid[r]*W + j]
   bool pat = false;
   int npat = 0, W = 0;
+  int wmax = 0; // entries of the longest row
   DeviceArray<uint8_t> pid;
   DeviceArray<int> ptab;
   // slot -> row when the rows are ordered by length in windows (SELL-C-sigma)
@@ -815,27 +816,33 @@ spmv(Context& c, const Level& L, const Sell& S, const TX* x, TO* y, const TO* b,
   const SellView<TV> A = view<TV>(S, sell_vals<TV>(S));
   const int nb = blocks_for(S.n, kRowThreads);
   const uint8_t* dm = L.dirmask.p;
+  if constexpr (MODE != kJacobi2) {
+    if (S.wmax > kPartMinWidth && S.n <= kPartMaxRows) {
+      launch(c,
+             S.pat   ? k_spmv_parts<MODE, TV, TX, TO, kColPat>
+             : A.c16 ? k_spmv_parts<MODE, TV, TX, TO, kColOff16>
+                     : k_spmv_parts<MODE, TV, TX, TO, kColIdx>,
+             S.nslices, kPartWarps * 32, A, x, y, b, dinv, dm, alpha, yidx, ystride, xcopy);
+      return;
+    }
+  }
   // FP32 values only: measured on C2, the FP32 cycle gains (1.550 -> 1.544 ms)
   // where the FP64 one, already at 64 registers for its smoother, loses
-  const bool small = sizeof(TV) == 4 && S.n < kSpmvSmallRows;
-  if (S.pat && small)
-    launch(c, k_spmv<MODE, TV, TX, TO, kColPat, true>, nb, kRowThreads, A, x, y, b, dinv,
-           dm, alpha, yidx, ystride, xcopy);
-  else if (S.pat)
-    launch(c, k_spmv<MODE, TV, TX, TO, kColPat>, nb, kRowThreads, A, x, y, b, dinv, dm,
-           alpha, yidx, ystride, xcopy);
-  else if (A.c16 && small)
-    launch(c, k_spmv<MODE, TV, TX, TO, kColOff16, true>, nb, kRowThreads, A, x, y, b, dinv,
-           dm, alpha, yidx, ystride, xcopy);
+  const bool few = sizeof(TV) == 4 && S.n < kSpmvSmallRows;
+  auto rows = [&](auto cm) {
+    constexpr int CM = decltype(cm)::value;
+    launch(c,
+           few                       ? k_spmv<MODE, TV, TX, TO, CM, kRowsFew>
+           : S.wmax > kPartMinWidth ? k_spmv<MODE, TV, TX, TO, CM, kRowsLong>
+                                    : k_spmv<MODE, TV, TX, TO, CM, kRowsWide>,
+           nb, kRowThreads, A, x, y, b, dinv, dm, alpha, yidx, ystride, xcopy);
+  };
+  if (S.pat)
+    rows(std::integral_constant<int, kColPat>{});
   else if (A.c16)
-    launch(c, k_spmv<MODE, TV, TX, TO, kColOff16>, nb, kRowThreads, A, x, y, b, dinv, dm,
-           alpha, yidx, ystride, xcopy);
-  else if (small)
-    launch(c, k_spmv<MODE, TV, TX, TO, kColIdx, true>, nb, kRowThreads, A, x, y, b, dinv,
-           dm, alpha, yidx, ystride, xcopy);
+    rows(std::integral_constant<int, kColOff16>{});
   else
-    launch(c, k_spmv<MODE, TV, TX, TO, kColIdx>, nb, kRowThreads, A, x, y, b, dinv, dm,
-           alpha, yidx, ystride, xcopy);
+    rows(std::integral_constant<int, kColIdx>{});
 }
 
 template<class T>

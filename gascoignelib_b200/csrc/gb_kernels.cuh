@@ -169,12 +169,30 @@ constexpr int kChunk = GB_SPMV_CHUNK;
 #define GB_SPMV_SMALL_ROWS 131072
 #endif
 constexpr int kSpmvSmallRows = GB_SPMV_SMALL_ROWS;
-template<int MODE, class TV, bool SMALL>
+// How a level's rows are loaded: kRowsWide, occupancy first; kRowsFew, levels
+// below kSpmvSmallRows; kRowsLong, rows of more than 32 entries, which come in
+// several chunks: more registers, so that a chunk's loads are in flight.
+enum RowShape
+{
+  kRowsWide = 0,
+  kRowsFew = 1,
+  kRowsLong = 2
+};
+// Blocks of 256 threads per SM for kRowsLong: FP32, the FP64 product, the other
+// FP64 modes. Measured on Q2 meshes, sweeps of 531,441 rows in FP32 with 8 / 6 /
+// 5 / 4: 43.3 / 43.5 / 40.7 / 45.1 us (64^3 Q1 with 5: 12.8 against 10.8 us);
+// the FP64 product with 8 / 6 / 5 / 4: 63.7 / 60.0 / 59.8 / 60.6 us, on 102,773
+// rows with hanging nodes 31.0 / 27.7 / 24.7 / 24.4 us; FP64 sweeps with 5 / 4 /
+// 3: 62.0 / 61.4 / 69.8 us.
+constexpr int kLongF32 = 5, kLongF64Ax = 5, kLongF64 = 4;
+template<int MODE, class TV, int SHAPE>
 constexpr int spmv_min_blocks()
 {
-  return SMALL ? 2
-               : (sizeof(TV) == 4 ? GB_SPMV_MINB_F32
-                                  : (MODE == 0 ? GB_SPMV_MINB_F64AX : GB_SPMV_MINB_F64));
+  if (SHAPE == kRowsFew)
+    return 2;
+  if (SHAPE == kRowsLong)
+    return sizeof(TV) == 4 ? kLongF32 : MODE == kAx ? kLongF64Ax : kLongF64;
+  return sizeof(TV) == 4 ? GB_SPMV_MINB_F32 : MODE == kAx ? GB_SPMV_MINB_F64AX : GB_SPMV_MINB_F64;
 }
 
 // Threads per CTA. The rows of a length window are sorted, so a CTA's warps
@@ -184,9 +202,9 @@ constexpr int spmv_min_blocks()
 // 23.1 / 20.2 / 20.9 us, 64^3 Q1 11.4 / 10.9 / 12.7 us; FP64, 80^3 Q2 65.0 /
 // 62.0 / 61.7 us.
 constexpr int kRowThreads = 128;
-template<int MODE, class TV, class TX, class TO, int CM, bool SMALL = false>
+template<int MODE, class TV, class TX, class TO, int CM, int SHAPE = kRowsWide>
 __global__ void __launch_bounds__(kRowThreads,
-                                  (spmv_min_blocks<MODE, TV, SMALL>() * 256 / kRowThreads))
+                                  (spmv_min_blocks<MODE, TV, SHAPE>() * 256 / kRowThreads))
 k_spmv(SellView<TV> A, const TX* __restrict__ x, TO* __restrict__ y,
        const TO* __restrict__ b, const TV* __restrict__ dinv,
        const uint8_t* __restrict__ dirmask, double alpha_,
@@ -259,6 +277,97 @@ k_spmv(SellView<TV> A, const TX* __restrict__ x, TO* __restrict__ y,
   } else { // kJacobi2: the second sweep on top of x1
     const TA h = static_cast<TA>(dinv[row]) * acc;
     y[row] = static_cast<TO>(x1(row) + alpha * h);
+  }
+}
+
+// k_spmv for long rows: kPartWarps warps (a CTA) share a slice and take its
+// columns in turn, four at a time (the 16-byte offset loads); a row's partial
+// sums are added in the warps' order. Which warp takes an entry depends on its
+// place in the row alone, so the slots' order leaves the result unchanged, but
+// the sum is not the sequential one of k_spmv: levels with rows of at most
+// kPartMinWidth entries, which the op programs of the multi-CTA cycle also run,
+// never take this form.
+constexpr int kPartWarps = 4;
+// Taken up to kPartMaxRows rows, where one thread per row leaves the GPU idle:
+// 9,261 Q2 rows with events around the launch: FP32 sweep 11.0 -> 8.9 us, FP64
+// product 15.6 -> 9.4 us. At 68,921 rows it is no faster (FP64 sweep 14.8 ->
+// 16.7 us), at 102,773 slower (28.0 -> 34.4 us).
+constexpr int kPartMinWidth = 32;
+constexpr int kPartMaxRows = 32768;
+template<int MODE, class TV, class TX, class TO, int CM>
+__global__ void __launch_bounds__(kPartWarps * 32, sizeof(TV) == 4 ? 10 : 8)
+k_spmv_parts(SellView<TV> A, const TX* __restrict__ x, TO* __restrict__ y,
+             const TO* __restrict__ b, const TV* __restrict__ dinv,
+             const uint8_t* __restrict__ dirmask, double alpha_,
+             const int* __restrict__ yidx, int64_t ystride, TX* __restrict__ xcopy)
+{
+  GB_PDL_ENTRY();
+  using TA = typename Acc<TV, TO>::type;
+  constexpr bool NEG = MODE == kResid || MODE == kResidDir || MODE == kJacobi;
+  constexpr int C = 16; // entries in flight
+  __shared__ TA part[kPartWarps][kSlice];
+  const int s = blockIdx.x, lane = threadIdx.x & 31, q = threadIdx.x >> 5;
+  const int slot = s * kSlice + lane;
+  const bool ok = slot < A.n;
+  const int row = !ok ? 0 : A.perm ? __ldg(A.perm + slot) : slot;
+  const int beg = A.sptr[s];
+  const int w = (A.sptr[s + 1] - beg) >> 5;
+  TA acc = TA(0);
+  if (ok) {
+    const TV* vp = A.val + beg + lane;
+    const int* cp = CM == kColPat ? (A.ptab + int(A.pid[row]) * A.W) : (A.col + beg + lane);
+    const int16_t* hp = A.c16 + beg + lane;
+    for (int j0 = 4 * q; j0 < w; j0 += C * kPartWarps) {
+      TA av[C], xv[C];
+      int4 o4;
+#pragma unroll
+      for (int k = 0; k < C; ++k) {
+        const int j = j0 + k / 4 * (4 * kPartWarps) + k % 4;
+        if (j < w) {
+          if (CM == kColPat && k % 4 == 0)
+            o4 = ldg(reinterpret_cast<const int4*>(cp + j));
+          const int c = CM == kColPat
+                          ? row + (k % 4 == 0 ? o4.x : k % 4 == 1 ? o4.y : k % 4 == 2 ? o4.z : o4.w)
+                          : CM == kColOff16 ? row + int(ldg(hp + j * kSlice))
+                                            : ldg(cp + j * kSlice);
+          av[k] = static_cast<TA>(ldg(vp + j * kSlice));
+          xv[k] = static_cast<TA>(ldg(x + c));
+        } else {
+          av[k] = TA(0);
+          xv[k] = TA(0);
+        }
+      }
+#pragma unroll
+      for (int k = 0; k < C; ++k)
+        acc = fma(av[k], xv[k], acc);
+    }
+  }
+  part[q][lane] = acc;
+  __syncthreads();
+  if (q != 0 || !ok)
+    return;
+#pragma unroll
+  for (int k = 1; k < kPartWarps; ++k)
+    acc += part[k][lane];
+  const TA alpha = static_cast<TA>(alpha_);
+  if (NEG)
+    acc = static_cast<TA>(b[row]) - acc;
+  if (yidx) {
+    const int64_t jj = *yidx;
+    xcopy[jj * ystride + row] = x[row];
+    y += (jj + 1) * ystride;
+  }
+  if (MODE == kAx) {
+    y[row] = static_cast<TO>(alpha * acc);
+  } else if (MODE == kAddAx) {
+    y[row] = static_cast<TO>(static_cast<TA>(y[row]) + alpha * acc);
+  } else if (MODE == kResid) {
+    y[row] = static_cast<TO>(acc);
+  } else if (MODE == kResidDir) {
+    y[row] = dirmask[row] ? TO(0) : static_cast<TO>(acc);
+  } else { // kJacobi: h = d*h; x = x + omega*h
+    const TA h = static_cast<TA>(dinv[row]) * acc;
+    y[row] = static_cast<TO>(static_cast<TA>(x[row]) + alpha * h);
   }
 }
 

@@ -61,6 +61,7 @@ build_sell(Sell& S, int64_t n, const int64_t* rowptr, const int64_t* col,
   S.n = static_cast<int>(n);
   S.nslices = static_cast<int>((n + kSlice - 1) / kSlice);
   S.nnz = rowptr[n];
+  S.wmax = 0;
   // the column patterns (per row, independent of the slot order)
   build_patterns(S, n, rowptr, col, st);
   // Slot order: on levels without column patterns (locality), rows in the
@@ -130,6 +131,7 @@ build_sell(Sell& S, int64_t n, const int64_t* rowptr, const int64_t* col,
     GB_REQUIRE(next < (int64_t(1) << 31), GB_EINVAL,
                "matrix too large for 32-bit SELL offsets");
     sptr[s + 1] = static_cast<int>(next);
+    S.wmax = std::max<int>(S.wmax, static_cast<int>(w));
   }
   S.entries = sptr[S.nslices];
   std::vector<int> c(S.entries);
