@@ -1077,15 +1077,21 @@ k_ilu_levels(int lv0, int lv1, const int* __restrict__ lptr, const int* __restri
 // of value 0 and a column that is always there (place chunk * B of the own
 // CTA, which holds zeros). A column is coded owner << 24 | place of its first
 // component; its block follows component-major.
+// Where a CTA's rows use few rows of other CTAs (a row goes to at most kIluPush
+// others), the CTA keeps copies of those behind its own (places chunk + 1 + k
+// for the k-th of its list ghost[gofs[r]..], ascending), which their owners
+// write (push: coded places, -1 none, kIluPush per slot); no column then is in
+// another CTA.
 template<class T>
 struct IluPack
 {
   int chunk;
-  const int *gptr, *row, *base, *col;
+  const int *gptr, *row, *base, *col, *push, *gofs;
   const T* val;
   const T* dinv; // backward only: the inverted diagonal blocks
 };
 
+constexpr int kIluPush = 2;
 constexpr int kIluOwnerShift = 24;
 constexpr int kIluPlaceMask = (1 << kIluOwnerShift) - 1;
 
@@ -1116,6 +1122,10 @@ struct IluWord<float>
   {
     asm volatile("st.relaxed.cluster.shared::cta.u32 [%0], %1;" ::"r"(a), "r"(v) : "memory");
   }
+  static __device__ __forceinline__ void send(uint32_t a, U v)
+  {
+    asm volatile("st.relaxed.cluster.shared::cluster.u32 [%0], %1;" ::"r"(a), "r"(v) : "memory");
+  }
 };
 template<>
 struct IluWord<double>
@@ -1139,6 +1149,10 @@ struct IluWord<double>
   {
     asm volatile("st.relaxed.cluster.shared::cta.u64 [%0], %1;" ::"r"(a), "l"(v) : "memory");
   }
+  static __device__ __forceinline__ void send(uint32_t a, U v)
+  {
+    asm volatile("st.relaxed.cluster.shared::cluster.u64 [%0], %1;" ::"r"(a), "l"(v) : "memory");
+  }
 };
 
 // entries consumed together: their blocks and y in registers
@@ -1156,6 +1170,7 @@ k_ilu_pack(int ngroups, int B, int chunk, const int* __restrict__ row,
            const int* __restrict__ base, const int* __restrict__ ptr,
            const int* __restrict__ fcol, const int* __restrict__ diag,
            const double* __restrict__ v, const int* __restrict__ gptr,
+           const int* __restrict__ gofs, const int* __restrict__ ghost,
            int* __restrict__ col, T* __restrict__ val, T* __restrict__ dinv)
 {
   GB_PDL_ENTRY();
@@ -1177,8 +1192,22 @@ k_ilu_pack(int ngroups, int B, int chunk, const int* __restrict__ row,
     const int p = UP ? first - (e - pad) : first + (e - pad);
     if (col) {
       const int k = e < pad ? 0 : fcol[p];
-      col[at * kSlice + lane] = e < pad ? (rank << kIluOwnerShift) | (chunk * B)
-                                        : ((k / chunk) << kIluOwnerShift) | ((k % chunk) * B);
+      int code = (rank << kIluOwnerShift) | (chunk * B);
+      if (e >= pad) {
+        code = ((k / chunk) << kIluOwnerShift) | ((k % chunk) * B);
+        if (k / chunk != rank && gofs[rank] < gofs[rank + 1]) {
+          int lo = gofs[rank], hi = gofs[rank + 1] - 1; // k is in the list
+          while (lo < hi) {
+            const int mid = (lo + hi) / 2;
+            if (ghost[mid] < k)
+              lo = mid + 1;
+            else
+              hi = mid;
+          }
+          code = (rank << kIluOwnerShift) | ((chunk + 1 + lo - gofs[rank]) * B);
+        }
+      }
+      col[at * kSlice + lane] = code;
     }
     for (int q = 0; q < B2; ++q)
       val[(at * B2 + q) * kSlice + lane] =
@@ -1190,9 +1219,14 @@ k_ilu_pack(int ngroups, int B, int chunk, const int* __restrict__ row,
         i < 0 ? T(0) : static_cast<T>(v[int64_t(d) * B2 + q]);
 }
 
-constexpr int kIluClusterThreads = 512;
+template<class T>
+__host__ __device__ constexpr int
+ilu_threads()
+{
+  return sizeof(T) == 4 ? 768 : 512;
+}
 constexpr size_t kIluClusterBytes = 216 * 1024; // of y in a CTA's shared memory
-constexpr int kIluGroupsPerLevel = 2;           // a CTA's share of an average level
+constexpr int kIluRowsPerLevel = 32; // a CTA's share of an average level
 
 // One direction of k_ilu_cluster: this CTA's groups, warp by warp in level
 // order. in: the rows' right-hand side; out: the result in global memory. All
@@ -1249,6 +1283,10 @@ ilu_cluster_run(const IluPack<T>& A, uint32_t y, int rank, const T* in, T* out, 
       for (int q = 0; q < B2; ++q)
         D[q] = __ldg(A.dinv + (int64_t(g) * B2 + q) * kSlice + lane);
     }
+    int push[kIluPush];
+#pragma unroll
+    for (int k = 0; k < kIluPush; ++k)
+      push[k] = A.push ? __ldg(A.push + (int64_t(g) * kIluPush + k) * kSlice + lane) : -1;
     T ui[UP ? B : 1];
     if (UP && u && !u_zero && i >= 0) {
 #pragma unroll
@@ -1344,6 +1382,20 @@ ilu_cluster_run(const IluPack<T>& A, uint32_t y, int rank, const T* in, T* out, 
         W::store(own + r * uint32_t(sizeof(T)), W::upper(w) == 0xffffffffu ? W::kNaN : w);
       }
 #pragma unroll
+      for (int k = 0; k < kIluPush; ++k)
+        if (push[k] >= 0) {
+          uint32_t a;
+          asm volatile("mapa.shared::cluster.u32 %0, %1, %2;"
+                       : "=r"(a)
+                       : "r"(y + uint32_t(push[k] & kIluPlaceMask) * uint32_t(sizeof(T))),
+                         "r"(push[k] >> kIluOwnerShift));
+#pragma unroll
+          for (int r = 0; r < B; ++r) {
+            const U w = W::bits(acc[r]);
+            W::send(a + r * uint32_t(sizeof(T)), W::upper(w) == 0xffffffffu ? W::kNaN : w);
+          }
+        }
+#pragma unroll
       for (int r = 0; r < B; ++r) {
         const int64_t k = int64_t(i) * B + r;
         out[k] = acc[r];
@@ -1366,19 +1418,20 @@ ilu_cluster_run(const IluPack<T>& A, uint32_t y, int rank, const T* in, T* out, 
 // with no barrier or launch between levels. A group's matrix entries are loaded
 // before it waits, so the other warps' loads run meanwhile. Each row runs
 // ilu_row's arithmetic in its order: the same bits. Measured on the 65^3 Q1
-// level (FP64, both substitutions): 0.65 ms against about 3.4 ms with the level
-// launches; a mixed solve of that mesh (6 steps) 112.9 -> 22.7 ms. About 0.42
-// us per level within one CTA, 0.72 us where levels cross CTAs. More warps hide
-// the matrix loads: 128 / 256 / 384 / 512 threads 1.81 / 0.98 / 0.74 / 0.65 ms
-// on the 65^3 level; two groups per average level and CTA (kIluGroupsPerLevel):
-// 1 / 2 / 4 measured 100 / 95 / 96 us on the 17^3 level, 225 / 232 / 282 us on
-// the 33^3 one. Levels whose y exceeds the cluster's shared memory (about
-// 440,000 rows in FP64, twice that in FP32) keep the level launches. Every wait
-// ends: a row
+// level (FP64, both substitutions): 0.57 ms against about 3.4 ms with the level
+// launches; a mixed solve of that mesh (6 steps) 112.9 -> 16.7 ms. About 0.42
+// us per level within one CTA. Reading other CTAs' memory in place of the copies
+// made it 0.65 ms (a group with one such column polls over the network). More
+// warps hide the matrix loads: 128 / 256 / 384 / 512 threads 1.81 / 0.98 / 0.74
+// / 0.65 ms in FP64, and in FP32, whose rows need 80 registers, 512 / 768
+// threads 18.8 / 16.7 ms for the solve. Rows of an average level per CTA
+// (kIluRowsPerLevel): 64 / 32 / 16 measured 213 / 183 / 180 us on the 33^3
+// level. Levels whose y exceeds the cluster's shared memory (about 440,000 rows
+// in FP64, twice that in FP32) keep the level launches. Every wait ends: a row
 // waits only for rows of earlier levels, a warp takes its groups in level
 // order, and the CTAs of a cluster run at the same time; bounded all the same.
 template<int B, class T>
-__global__ void __launch_bounds__(kIluClusterThreads, 1)
+__global__ void __launch_bounds__(ilu_threads<T>(), 1)
 k_ilu_cluster(IluPack<T> lo, IluPack<T> up, int n, const T* rhs, T* h, T* u, double omega,
               int u_zero, int* err, unsigned long long wait_ns)
 {
@@ -1388,21 +1441,24 @@ k_ilu_cluster(IluPack<T> lo, IluPack<T> up, int n, const T* rhs, T* h, T* u, dou
   uint32_t rank;
   asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
   const uint32_t y = static_cast<uint32_t>(__cvta_generic_to_shared(ilu_smem));
-  const int mine = min(lo.chunk, n - int(rank) * lo.chunk) * B;
-  auto mark = [&]() {
+  const int mine = min(lo.chunk, n - int(rank) * lo.chunk) * B, copies = (lo.chunk + 1) * B;
+  auto mark = [&](const IluPack<T>& A) {
     for (int k = threadIdx.x; k < mine; k += blockDim.x)
       W::store(y + uint32_t(k) * uint32_t(sizeof(T)), W::kMark);
+    const int nc = (A.gofs[rank + 1] - A.gofs[rank]) * B;
+    for (int k = threadIdx.x; k < nc; k += blockDim.x)
+      W::store(y + uint32_t(copies + k) * uint32_t(sizeof(T)), W::kMark);
   };
   if (threadIdx.x == 0)
     give_up = 0;
   if (threadIdx.x < B) // what the entries before a row's first one read
     W::store(y + uint32_t(lo.chunk * B + threadIdx.x) * uint32_t(sizeof(T)), 0);
-  mark();
   GB_PDL_ENTRY();
+  mark(lo);
   cluster_barrier();
   ilu_cluster_run<B, T, false>(lo, y, int(rank), rhs, h, nullptr, T(0), false, &give_up, wait_ns);
   cluster_barrier();
-  mark();
+  mark(up);
   cluster_barrier();
   ilu_cluster_run<B, T, true>(up, y, int(rank), h, h, u, static_cast<T>(omega), u_zero != 0,
                               &give_up, wait_ns);

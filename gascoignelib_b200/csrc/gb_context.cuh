@@ -300,6 +300,8 @@ struct Level
   // and backward 1; ctas 0: the level's rows do not fit a cluster
   int ilu_ctas = 0, ilu_chunk = 0, ilu_groups[2] = { 0, 0 };
   DeviceArray<int> ilu_gptr[2], ilu_grow[2], ilu_gbase[2], ilu_gcol[2];
+  DeviceArray<int> ilu_push[2], ilu_gofs[2], ilu_ghost[2]; // copies of other CTAs' rows
+  int ilu_places = 0; // of y in a CTA's shared memory, in rows
   DeviceArray<double> ilu_gval64[2], ilu_gdinv64;
   DeviceArray<float> ilu_gval32[2], ilu_gdinv32;
   // values assembled on the device since the host copy was made
@@ -749,7 +751,7 @@ template<class T>
 inline bool
 ilu_in_cluster(const Context& c, const Level& L)
 {
-  return L.ilu_ctas > 0 && size_t(L.ilu_chunk) * L.B * sizeof(T) <= kIluClusterBytes;
+  return L.ilu_ctas > 0 && size_t(L.ilu_places) * L.B * sizeof(T) <= kIluClusterBytes + 32;
 }
 void ensure_work(Context& c);
 

@@ -316,7 +316,8 @@ ilu_pack_of(const Level& L, int dir)
   const void* dinv = sizeof(T) == 8 ? static_cast<const void*>(L.ilu_gdinv64.p)
                                     : static_cast<const void*>(L.ilu_gdinv32.p);
   return IluPack<T>{ L.ilu_chunk, L.ilu_gptr[dir].p, L.ilu_grow[dir].p, L.ilu_gbase[dir].p,
-                     L.ilu_gcol[dir].p, static_cast<const T*>(val),
+                     L.ilu_gcol[dir].p, L.ilu_push[dir].p, L.ilu_gofs[dir].p,
+                     static_cast<const T*>(val),
                      static_cast<const T*>(dinv) };
 }
 
@@ -326,11 +327,11 @@ void Emit<T>::ilu_cluster(int l, const T* rhs, T* h, T* u, bool u_zero)
   const Level& L = c.L[l];
   no_rec();
   auto run = [&](auto* kern) {
-    const size_t smem = (size_t(L.ilu_chunk) + 1) * L.B * sizeof(T);
+    const size_t smem = size_t(L.ilu_places) * L.B * sizeof(T);
     GB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
     GB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  int(kIluClusterBytes + 32)));
-    launch_cluster(c, kern, L.ilu_ctas, kIluClusterThreads, int(smem), ilu_pack_of<T>(L, 0),
+    launch_cluster(c, kern, L.ilu_ctas, ilu_threads<T>(), int(smem), ilu_pack_of<T>(L, 0),
                    ilu_pack_of<T>(L, 1), (int)L.n, rhs, h, u, c.params.omega, int(u_zero),
                    c.miderr.p, c.wait_ns);
   };

@@ -843,7 +843,7 @@ ilu_groups(Context& c, Level& L, const std::vector<int> (&lev)[2], const int (&n
   if (!c.ilu_cluster || (n + 1) * L.B >= (int64_t(1) << kIluOwnerShift))
     return;
   if (!c.ilu_max_ctas)
-    c.ilu_max_ctas = max_ctas(k_ilu_cluster<1, double>, kIluClusterThreads, kIluClusterBytes + 32);
+    c.ilu_max_ctas = max_ctas(k_ilu_cluster<1, double>, ilu_threads<double>(), kIluClusterBytes + 32);
   const int most = c.ilu_max_ctas;
   auto bytes = [&](int ctas, size_t size) { return size_t((n + ctas - 1) / ctas) * L.B * size; };
   const size_t size = bytes(most, 8) <= kIluClusterBytes ? 8 : 4;
@@ -852,9 +852,50 @@ ilu_groups(Context& c, Level& L, const std::vector<int> (&lev)[2], const int (&n
   int ctas = 1;
   while (ctas < most &&
          (bytes(ctas, size) > kIluClusterBytes ||
-          n > int64_t(ctas) * nlev[0] * kIluGroupsPerLevel * kSlice))
+          n > int64_t(ctas) * nlev[0] * kIluRowsPerLevel))
     ctas *= 2;
   const int chunk = static_cast<int>((n + ctas - 1) / ctas), half = ilu_half(L.B);
+  // the rows of other CTAs that each CTA uses, and where each row is used
+  std::vector<int> gofs[2], ghost[2], push[2];
+  int copies = 0;
+  bool pushed = ctas > 1;
+  for (int dir = 0; dir < 2 && pushed; ++dir) {
+    push[dir].assign(size_t(n) * kIluPush, -1);
+    gofs[dir].assign(1, 0);
+    for (int r = 0; r < ctas && pushed; ++r) {
+      const int64_t i0 = int64_t(r) * chunk, i1 = std::min<int64_t>(n, i0 + chunk);
+      std::vector<int> used;
+      for (int64_t i = i0; i < i1; ++i)
+        for (int p = dir ? diag[i] + 1 : ptr[i]; p < (dir ? ptr[i + 1] : diag[i]); ++p)
+          if (col[p] < i0 || col[p] >= i1)
+            used.push_back(col[p]);
+      std::sort(used.begin(), used.end());
+      used.erase(std::unique(used.begin(), used.end()), used.end());
+      for (size_t k = 0; k < used.size() && pushed; ++k) {
+        int* at = push[dir].data() + size_t(used[k]) * kIluPush;
+        int q = 0;
+        while (q < kIluPush && at[q] >= 0)
+          ++q;
+        pushed = q < kIluPush;
+        if (pushed)
+          at[q] = (r << kIluOwnerShift) | ((chunk + 1 + int(k)) * L.B);
+      }
+      ghost[dir].insert(ghost[dir].end(), used.begin(), used.end());
+      gofs[dir].push_back(static_cast<int>(ghost[dir].size()));
+      copies = std::max(copies, static_cast<int>(used.size()));
+    }
+  }
+  // not where a row goes to many CTAs or the copies do not fit
+  if (!pushed || size_t(chunk + 1 + copies) * L.B * size > kIluClusterBytes ||
+      int64_t(chunk + 1 + copies) * L.B >= (int64_t(1) << kIluOwnerShift)) {
+    copies = 0;
+    pushed = false;
+    for (int dir = 0; dir < 2; ++dir) {
+      gofs[dir].assign(ctas + 1, 0);
+      ghost[dir].clear();
+    }
+  }
+  L.ilu_places = chunk + 1 + copies;
   for (int dir = 0; dir < 2; ++dir) {
     // rows sorted by (owner, level), ascending within: a counting sort
     const int nl = nlev[dir];
@@ -881,7 +922,7 @@ ilu_groups(Context& c, Level& L, const std::vector<int> (&lev)[2], const int (&n
             const int b = dir ? diag[i] + 1 : ptr[i], e = dir ? ptr[i + 1] : diag[i];
             w = std::max(w, (e - b + half - 1) / half * half);
             if (e > b) // ascending columns: the first and the last tell
-              far = far || col[b] / chunk != r || col[e - 1] / chunk != r;
+              far = far || (!pushed && (col[b] / chunk != r || col[e - 1] / chunk != r));
           }
           GB_REQUIRE(int64_t(base.back() >> 1) + w < (int64_t(1) << 30), GB_EINVAL,
                      "ILU groups too large");
@@ -897,6 +938,23 @@ ilu_groups(Context& c, Level& L, const std::vector<int> (&lev)[2], const int (&n
     GB_CUDA(L.ilu_grow[dir].alloc(row.size()));
     GB_CUDA(L.ilu_gbase[dir].alloc(base.size()));
     GB_CUDA(L.ilu_gcol[dir].alloc(std::max<size_t>(cols, 1)));
+    GB_CUDA(L.ilu_gofs[dir].alloc(gofs[dir].size()));
+    GB_CUDA(L.ilu_ghost[dir].alloc(std::max<size_t>(ghost[dir].size(), 1)));
+    GB_CUDA(h2d(c.stream, L.ilu_gofs[dir].p, gofs[dir].data(), gofs[dir].size() * sizeof(int)));
+    if (!ghost[dir].empty())
+      GB_CUDA(h2d(c.stream, L.ilu_ghost[dir].p, ghost[dir].data(),
+                  ghost[dir].size() * sizeof(int)));
+    if (pushed) { // per slot, in the groups' order
+      std::vector<int> to(row.size() * kIluPush, -1);
+      for (size_t k = 0; k < row.size(); ++k)
+        for (int q = 0; q < kIluPush && row[k] >= 0; ++q)
+          to[(k / kSlice * kIluPush + q) * kSlice + k % kSlice] =
+            push[dir][size_t(row[k]) * kIluPush + q];
+      GB_CUDA(L.ilu_push[dir].alloc(to.size()));
+      GB_CUDA(h2d(c.stream, L.ilu_push[dir].p, to.data(), to.size() * sizeof(int)));
+    } else {
+      L.ilu_push[dir].release();
+    }
     GB_CUDA(L.ilu_gval32[dir].alloc(std::max<size_t>(cols * B2, 1)));
     if (size == 8)
       GB_CUDA(L.ilu_gval64[dir].alloc(std::max<size_t>(cols * B2, 1)));
@@ -926,7 +984,8 @@ ilu_pack(Context& c, Level& L)
       launch(c, kern, nb, 256, ng, L.B, L.ilu_chunk, (const int*)L.ilu_grow[dir].p,
              (const int*)L.ilu_gbase[dir].p, (const int*)L.ilu_ptr.p, (const int*)L.ilu_col.p,
              (const int*)L.ilu_diag.p, (const double*)L.ilu_v64.p,
-             (const int*)L.ilu_gptr[dir].p, col, val, dinv);
+             (const int*)L.ilu_gptr[dir].p, (const int*)L.ilu_gofs[dir].p,
+             (const int*)L.ilu_ghost[dir].p, col, val, dinv);
     };
     int* col = L.ilu_gcol[dir].p;
     if (dir)

@@ -33,6 +33,20 @@ def _blocks_of_two(n):
     return Problem(dim=2, levels=[level], transfers=[], rhs=rng.uniform(-1, 1, 2 * n))
 
 
+def _scattered(n):
+    """One level whose rows use rows of many other CTAs (no copies of those then)."""
+    rng = np.random.default_rng(6)
+    rows = [sorted({i, *rng.integers(0, n, size=5).tolist()}) for i in range(n)]
+    ptr = np.concatenate([[0], np.cumsum([len(r) for r in rows])]).astype(np.int64)
+    col = np.concatenate(rows).astype(np.int64)
+    diag = np.array([ptr[i] + r.index(i) for i, r in enumerate(rows)], dtype=np.int64)
+    val = rng.uniform(-1.0, 1.0, size=col.size)
+    val[diag] = 8.0
+    level = Level(n=n, B=1, rowptr=ptr, col=col, diag=diag, val=val,
+                  dirichlet=np.array([0], dtype=np.int64))
+    return Problem(dim=2, levels=[level], transfers=[], rhs=rng.uniform(-1, 1, n))
+
+
 CASES = {
     "2d_4": lambda: _diffusion(2, 2, 1),
     "2d_96": lambda: _diffusion(2, 3, 5),
@@ -41,6 +55,7 @@ CASES = {
     "q2_3d_12": lambda: structured_q2(3, 3, 2),
     "stokes_2d": lambda: structured_stokes(2, 3, 3),
     "stokes_3d": lambda: structured_stokes(3, 2, 2),
+    "scattered_20000": lambda: _scattered(20000),
     "blocks_of_two_1": lambda: _blocks_of_two(1),
     "blocks_of_two_333": lambda: _blocks_of_two(333),
 }
