@@ -68,7 +68,6 @@ assemble_level(Context& c, int l, const double* beta)
                                              : c.asm_E.alloc(size_t(nc) * nl * nl));
   const double b0 = beta ? beta[0] : 0.0, b1 = beta ? beta[1] : 0.0;
   const double b2 = beta && dim == 3 ? beta[2] : 0.0;
-  const double g = 0.5 / std::sqrt(3.0);
   const bool conv = b0 != 0.0 || b1 != 0.0 || b2 != 0.0;
   L.m_beta[0] = b0;
   L.m_beta[1] = b1;
@@ -78,7 +77,7 @@ assemble_level(Context& c, int l, const double* beta)
   L.m_assembled = true;
 #define GB_ELEM(D, CV)                                                                   \
   launch(c, k_q1_element<D, CV>, blocks_for(nc, 128), 128, nc, (const int*)L.m_cells.p,  \
-         (const double*)L.m_coords.p, (const double*)L.m_kappa.p, b0, b1, b2, g, c.asm_E.p)
+         (const double*)L.m_coords.p, (const double*)L.m_kappa.p, b0, b1, b2, c.asm_E.p)
   GB_REQUIRE(c.lps_s0 == 0.0 || L.mesh_deg >= 2, GB_EINVAL,
              "LPS is built for patch elements only (Q2, or Q1 on patches)");
   const bool lps = conv && c.lps_s0 > 0.0;
@@ -178,7 +177,6 @@ form_level(Context& c, int l, double* y, double* x, double d)
   const int nc = static_cast<int>(L.mesh_ncells);
   const double b0 = L.m_beta[0], b1 = L.m_beta[1], b2 = L.m_beta[2];
   const bool conv = b0 != 0.0 || b1 != 0.0 || b2 != 0.0;
-  const double g = 0.5 / std::sqrt(3.0);
   Emit<double> Em{ c, nullptr };
   if (L.has_hn())
     Em.hn_average(l, x);
@@ -186,7 +184,7 @@ form_level(Context& c, int l, double* y, double* x, double d)
   if (L.mesh_deg == 1) {
 #define GB_FORM(D, CV)                                                                 \
   launch(c, k_q1_form<D, CV>, blocks_for(nc, 128), 128, nc, (const int*)L.m_cells.p,   \
-         (const double*)L.m_coords.p, (const double*)L.m_kappa.p, b0, b1, b2, g,        \
+         (const double*)L.m_coords.p, (const double*)L.m_kappa.p, b0, b1, b2,           \
          (const double*)x, c.asm_R.p)
     if (dim == 2) {
       if (conv) GB_FORM(2, true); else GB_FORM(2, false);
