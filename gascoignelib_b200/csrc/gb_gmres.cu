@@ -648,14 +648,16 @@ fgmres_graph(Context& c, double* x, const double* b, int prec, gb_solve_info* in
 // ------------------------------------------- left-preconditioned, one graph
 //
 // The same solver for gmressize <= kCgsMaxJ: the Arnoldi loop as a conditional
-// WHILE node, with no host round trip per step, and the basis orthogonalised by
-// the two CGS passes of the flexible solver (two launches per step) instead of
-// one launch per basis vector. CGS2 leaves the basis as orthogonal as modified
-// Gram-Schmidt with its second pass does, so the reference's test for a second
-// pass never asks for one; H and the residuals agree to rounding, and CGInfo's
-// rule ends the loop as before. A step of a 129^2 Q1 problem (18 steps) was 35
-// launches in 158 us, half of it Gram-Schmidt and the host's read of the flags;
-// it is 26 in 80 us (the solve 2.80 -> 1.54 ms; 57^3 Q1, 12 steps: 2.58 -> 1.88).
+// WHILE node, with no host round trip per step, and modified Gram-Schmidt in two
+// launches per step instead of one per basis vector: d_i = <w - sum_{k<i} d_k
+// V_k, V_i> = <w, V_i> - sum_{k<i} d_k <V_k, V_i>, the basis' own dots being at
+// hand from the pass that formed each vector (k_cgs with kStepCgInfo). It is the
+// reference's one pass, not a re-orthogonalised one: at a breakdown, where the
+// next vector is rounding noise, CGInfo ends the loop at the same step. (The
+// reference repeats the pass only for a vector of norm 0, which stays 0.) A step
+// of a 129^2 Q1 problem (18 steps) was 35 launches in 158 us, half of it
+// Gram-Schmidt and the host's read of the flags; it is 26 in 80 us (the solve
+// 2.80 -> 1.54 ms; 57^3 Q1, 12 steps: 2.58 -> 1.88).
 void
 left_setup(Context& c, cudaGraphConditionalHandle hLoop, int use_cond)
 {
@@ -683,9 +685,8 @@ left_step(Context& c, cudaGraphConditionalHandle hLoop, int use_cond)
   const int64_t n = L.ndof();
   GmresDev* G = c.G.p;
   double* V = c.krylov.p;
-  // v_j (the last step's second pass and scaling applied), p = A v_j, w = M p
-  launch(c, k_load_idx<double>, stream_blocks(n), 256, n, c.rhs64.p, V, (const GmresDev*)G,
-         (const double*)nullptr, (double*)nullptr, 0.0);
+  // v_j (the last step's vector scaled), p = A v_j, w = M p
+  launch(c, k_load_scaled, stream_blocks(n), 256, n, c.rhs64.p, V, (const GmresDev*)G);
   spmv<kAx, double, double, double>(c, L, opA(c, L), (const double*)c.rhs64.p, c.pbuf.p, nullptr,
                                     nullptr, 1.0);
   precondition_T<double>(c, c.w64, c.zfix64.p, c.pbuf.p, true);

@@ -1004,6 +1004,7 @@ struct GmresDev
   int reached, need_reortho, zero_rho, pad;
   // graph-resident flexible GMRES
   double d2[kMaxV + 1];       // second CGS pass coefficients
+  double gram[32][32];        // <V_k, V_i>, k < i (left-preconditioned solver)
   double beta_tmp;            // ||r|| of the current restart
   int j;                      // Arnoldi step of the current cycle
   int total;                  // Arnoldi steps over all cycles
@@ -1296,6 +1297,24 @@ k_load_idx(int64_t n, TO* __restrict__ y, double* __restrict__ V,
   }
 }
 
+// v_j = v_j / s (j > 0: the previous step left w' there) and a copy of it.
+static __global__ void __launch_bounds__(256)
+k_load_scaled(int64_t n, double* __restrict__ y, double* __restrict__ V,
+              const GmresDev* __restrict__ G)
+{
+  GB_PDL_ENTRY();
+  const int j = G->j;
+  const double s = j ? G->inv : 1.0;
+  double* v = V + int64_t(j) * n;
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n;
+       i += (int64_t)gridDim.x * blockDim.x) {
+    const double t = s * v[i];
+    if (j)
+      v[i] = t;
+    y[i] = t;
+  }
+}
+
 // V[(*jp) * n + i] *= *s
 static __global__ void
 k_scale_idx(int64_t n, double* __restrict__ V, const int* __restrict__ jp,
@@ -1310,7 +1329,10 @@ k_scale_idx(int64_t n, double* __restrict__ V, const int* __restrict__ jp,
 }
 
 // Classical Gram-Schmidt, twice (CGS2), on w = V_{j+1} against V_0..V_j, j = G->j
-// (pass 0 reads w from src0 when that is set, and stores it):
+// (pass 0 reads w from src0 when that is set, and stores it). With kStepCgInfo
+// the two passes are one modified Gram-Schmidt pass instead: pass 0 corrects its
+// dots by the basis' own (gram), pass 1 subtracts and forms ||w'|| and, from its
+// dots, the new vector's gram entries; there is no second update:
 //  MODE 0: c1[i] = <w, V_i>;                         H[j][i]  = c1[i]
 //  MODE 1: w -= sum_i c1[i] V_i; c2[i] = <w, V_i>;   H[j][i] += c2[i]
 //  MODE 2: w -= sum_i c2[i] V_i; s = ||w||;          H[j][j+1] = s
@@ -1489,7 +1511,20 @@ k_cgs(int64_t n, double* __restrict__ V, const double* src0, GmresDev* G, double
   // one thread per coefficient; only the rotations, a recurrence, run on one
   // thread, on copies in shared memory
   if (MODE == 0) {
-    if (tid < nv) {
+    if (rule == kStepCgInfo && wid == 0) {
+      // modified Gram-Schmidt's coefficients from the plain dots and the basis'
+      // own dots: d_i = <w - sum_{k<i} d_k V_k, V_i>
+      double a = lane < nv ? s_red[lane] : 0.0;
+      for (int k = 0; k + 1 < nv; ++k) {
+        const double g = lane > k && lane < nv ? G->gram[k][lane] : 0.0;
+        const double dk = __shfl_sync(0xffffffffu, a, k);
+        a = fma(-dk, g, a);
+      }
+      if (lane < nv)
+        s_red[lane] = a;
+      __syncwarp();
+    }
+    if (tid < nv) { // nv <= 32: the same warp
       G->d[tid] = s_red[tid];
       G->H[j][tid] = s_red[tid];
     }
@@ -1499,7 +1534,7 @@ k_cgs(int64_t n, double* __restrict__ V, const double* src0, GmresDev* G, double
   }
   if (MODE == 1 && tid < nv) {
     G->d2[tid] = s_red[tid];
-    s_h[tid] = G->H[j][tid] + s_red[tid];
+    s_h[tid] = G->H[j][tid] + (rule == kStepCgInfo ? 0.0 : s_red[tid]);
   }
   if (tid < j) {
     s_ci[tid] = G->ci[tid];
@@ -1510,7 +1545,7 @@ k_cgs(int64_t n, double* __restrict__ V, const double* src0, GmresDev* G, double
     double sv;
     if (MODE == 1) {
       double c2 = 0.0;
-      for (int i = 0; i < nv; ++i)
+      for (int i = 0; i < nv && rule != kStepCgInfo; ++i)
         c2 = fma(s_red[i], s_red[i], c2);
       sv = sqrt(fmax(s_red[nv] - c2, 0.0));
     } else {
@@ -1524,6 +1559,8 @@ k_cgs(int64_t n, double* __restrict__ V, const double* src0, GmresDev* G, double
     arnoldi_step(G, s_h, s_ci, s_si, inner, m, use_cond, rule);
   }
   __syncthreads();
+  if (rule == kStepCgInfo && tid < nv && nv < kCgsMaxJ) // <V_tid, V_{j+1}>
+    G->gram[tid][nv] = s_red[tid] / G->s;
   if (tid <= nv)
     G->H[j][tid] = s_h[tid];
 }
