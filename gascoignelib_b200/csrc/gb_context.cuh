@@ -409,6 +409,7 @@ struct gb_ctx
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
     int64_t version = -1;
+    int64_t seen = -1; // the version of the last solve (left solver)
     int setup_k = 0, outer_k = 0, inner_k = 0;
   } fg[2][2]; // [operator transposed][cycle precision]
   FGraph lg[2]; // the left-preconditioned solver's, [operator transposed]

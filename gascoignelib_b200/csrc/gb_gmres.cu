@@ -778,14 +778,22 @@ gmres_left(Context& c, double* x, const double* b, gb_solve_info* info)
     return gmres_left_mgs(c, x, b, info);
   left_buffers(c);
   auto& LG = c.lg[c.transposed];
-  if (c.use_graph && (!LG.exec || LG.version != c.version))
+  // A program may solve once per matrix (a Newton step that uploads new values):
+  // building the graph (about 2 ms) takes longer than the launches it saves in
+  // one solve, so it is built by the second solve with the same levels and keys.
+  // Both ways give the same bits.
+  bool graph = c.use_graph && LG.exec && LG.version == c.version;
+  if (c.use_graph && !graph && LG.seen == c.version) {
     build_left_graph(c);
+    graph = true;
+  }
+  LG.seen = c.version;
   const int64_t n = c.L[c.nlevels - 1].ndof();
   GB_CUDA(cudaMemcpyAsync(c.bg.p, b, n * sizeof(double), cudaMemcpyDeviceToDevice, c.stream));
   const int64_t l0 = c.launches;
   GB_CUDA(cudaEventRecord(c.ev0, c.stream));
   GB_CUDA(cudaMemsetAsync(c.G.p, 0, sizeof(GmresDev), c.stream));
-  if (c.use_graph) {
+  if (graph) {
     GB_CUDA(cudaGraphLaunch(LG.exec, c.stream));
   } else {
     left_setup(c, 0, 0);
@@ -807,7 +815,7 @@ gmres_left(Context& c, double* x, const double* b, gb_solve_info* info)
     fill_info_enqueue(c, c.xg.p, c.bg.p);
   GB_CUDA(cudaStreamSynchronize(c.stream));
   int64_t kernels = c.launches - l0;
-  if (c.use_graph) {
+  if (graph) {
     const int64_t in_graph = LG.setup_k + int64_t(st[3]) * LG.inner_k;
     c.launches += in_graph;
     kernels += in_graph;
