@@ -394,7 +394,7 @@ bool Emit<T>::exact_sweeps(int l, int niter, T* u, const T* b, bool u_zero)
                                int(kExactBytes)));
   launch_cluster(c, k_exact_sweeps<T>, ctas, kExactWarps * 32, int(smem),
                  view<T>(A, sell_vals<T>(A)), slices, parts, niter, int(u_zero), b,
-                 dinv_of<T>(L), u, c.params.omega, c.miderr.p, c.wait_ns);
+                 dinv_of<T>(L), u, c.params.omega);
   return true;
 }
 

@@ -2013,17 +2013,25 @@ cluster_barrier()
 // of a few thousand rows as a launch of its own is latency only (launch, then
 // range, column and x one after the other: 8 to 17 us for 3,375 rows of 27 or
 // 1,331 rows of up to 125 entries). Here each CTA copies its slices (`slices`
-// each) to shared memory once, with 16-bit columns, and keeps all of x; after a
+// each) to shared memory once, with 16-bit columns, and keeps all of x; in a
 // sweep each CTA sends its new values into every CTA's copy over the cluster
-// network, each store counted on the receiver's mbarrier, and a sweep starts
-// when all n values of the last one have come (a cluster barrier per sweep
-// instead: 2 us more for 9 sweeps). Measured on 16 CTAs, 9 sweeps with events
-// around the launch: 27 us for 1,331 Q2 rows in FP32, 37 us in FP64, 25 us for
-// 3,375 Q1 rows in FP64; 8 CTAs 6 to 8 us more. Solves of 80^3 Q2 cells 51.1 ->
-// 46.3 ms, 40^3 Q2 cells with a refined ball 51.9 -> 46.6 ms, 56^3 Q1 cells
-// (left) 2.32 -> 2.28 ms. Two copies and two mbarriers take turns: a CTA
-// sends sweep k + 2 only after it has every CTA's k + 1, which that CTA sent
-// after its last read of k's copy and after its wait for k. `parts`
+// network, and the cluster's hardware barrier (release/acquire at cluster scope)
+// ends the sweep. Measured on 16 CTAs, 9 sweeps with events around the launch:
+// 29 us for 1,331 Q2 rows in FP32, 38 us in FP64, 31 us for 3,375 Q1 rows in
+// FP64; 8 CTAs 6 to 8 us more. (Counting every value on the receiver's mbarrier
+// in place of the barrier: 27, 37 and 29 us, but nothing then tells a CTA that is
+// ahead that another CTA's threads have read their partial sums, and a wait that
+// ran out would leave values under way.) Solves against a launch per sweep: 80^3
+// Q2 cells 51.1 -> 46.5 ms, 40^3 Q2 cells with a refined ball 51.9 -> 46.9 ms.
+// Why nothing is overwritten while it is read: a sweep's last reads of `part`
+// and of the old copy of x come before its cluster barrier, for every thread of
+// every CTA, and the next sweep, which is the next to write `part` and the old
+// copy, begins after it. Within a sweep `part` is written before the
+// __syncthreads and read after it, and values are sent into the other copy, which
+// nobody reads before the barrier. A thread may thus send to some of the CTAs
+// only (`sub`): all of them wait for it. No wait here can run out: a cluster is
+// co-scheduled as a whole, every thread reaches every barrier, and the last
+// barrier lies after the last access to another CTA's memory. `parts`
 // warps share a slice: each takes every parts-th entry of its 32 rows, and a
 // row's partial sums are added in the warps' order, so the order is not the
 // sequential kernel's. x holds the start (zero: from 0, the first sweep needs
@@ -2041,30 +2049,28 @@ exact_smem(int64_t n, int64_t entries, int slices, int parts)
          size_t(entries) * (sizeof(T) + 2);
 }
 
-// The value v to shared address a of CTA r, counted on that CTA's mbarrier.
+// The value v to shared address a of CTA r.
 template<class T>
 __device__ __forceinline__ void
-send_counted(uint32_t a, uint32_t mbar, uint32_t r, T v)
+send_to_cta(uint32_t a, uint32_t r, T v)
 {
-  uint32_t ra, rm;
+  uint32_t ra;
   asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(ra) : "r"(a), "r"(r));
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(rm) : "r"(mbar), "r"(r));
   if (sizeof(T) == 8)
-    asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.b64 [%0], %1, [%2];"
-                 ::"r"(ra), "l"(__double_as_longlong(double(v))), "r"(rm) : "memory");
+    asm volatile("st.shared::cluster.b64 [%0], %1;"
+                 ::"r"(ra), "l"(__double_as_longlong(double(v))) : "memory");
   else
-    asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.b32 [%0], %1, [%2];"
-                 ::"r"(ra), "r"(__float_as_uint(float(v))), "r"(rm) : "memory");
+    asm volatile("st.shared::cluster.b32 [%0], %1;"
+                 ::"r"(ra), "r"(__float_as_uint(float(v))) : "memory");
 }
 
 template<class T>
 __global__ void __launch_bounds__(kExactWarps * 32, 1)
 k_exact_sweeps(SellView<T> A, int slices, int parts, int niter, int zero,
                const T* __restrict__ b, const T* __restrict__ dinv, T* __restrict__ x,
-               double omega_, int* err, unsigned long long wait_ns)
+               double omega_)
 {
   extern __shared__ __align__(16) unsigned char exact_sm[];
-  __shared__ __align__(8) unsigned long long came[2];
   constexpr int kThreads = kExactWarps * 32;
   const int n = A.n, np = n + (n & 1), nsl = (n + kSlice - 1) / kSlice;
   uint32_t rank, ctas;
@@ -2112,20 +2118,10 @@ k_exact_sweeps(SellView<T> A, int slices, int parts, int niter, int zero,
   }
   for (int i = threadIdx.x; i < n; i += kThreads)
     xs[i] = zero ? omega * (__ldg(dinv + i) * __ldg(b + i)) : x[i];
-  const uint32_t bar = static_cast<uint32_t>(__cvta_generic_to_shared(came));
-  if (threadIdx.x == 0) {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar));
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar + 8));
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-  }
   cluster_barrier(); // every CTA has read x, and is there to be written to
   const uint32_t xbase = static_cast<uint32_t>(__cvta_generic_to_shared(xs));
-  int cur = 0, turn = 0;
-  for (int it = zero ? 1 : 0; it < niter; ++it, ++turn) {
-    const uint32_t mbar = bar + 8 * (turn & 1);
-    if (threadIdx.x == 0)
-      asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;"
-                   ::"r"(mbar), "r"(uint32_t(n) * uint32_t(sizeof(T))) : "memory");
+  int cur = 0;
+  for (int it = zero ? 1 : 0; it < niter; ++it) {
     const T* xo = xs + cur * np;
     if (work) {
       T acc = T(0);
@@ -2145,27 +2141,11 @@ k_exact_sweeps(SellView<T> A, int slices, int parts, int niter, int zero,
       const T v = xo[urow] + omega * (dr * (br - acc));
       const uint32_t a = xbase + uint32_t((1 - cur) * np + urow) * uint32_t(sizeof(T));
       for (uint32_t r = sub; r < ctas; r += share)
-        send_counted<T>(a, mbar, r, v);
+        send_to_cta<T>(a, r, v);
     }
-    // all n values of this sweep (bounded: the wait always ends)
-    const uint32_t phase = (turn >> 1) & 1;
-    const unsigned long long t0 = global_ns();
-    for (;;) {
-      uint32_t done;
-      asm volatile("{\n\t.reg .pred p;\n\t"
-                   "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
-                   "selp.u32 %0, 1, 0, p;\n\t}"
-                   : "=r"(done) : "r"(mbar), "r"(phase) : "memory");
-      if (done)
-        break;
-      if (global_ns() - t0 > wait_ns) {
-        atomicExch(err, 1);
-        break;
-      }
-    }
+    cluster_barrier();
     cur = 1 - cur;
   }
-  cluster_barrier(); // nothing is under way to a CTA that has left
   if (upd && sub == 0)
     x[urow] = xs[cur * np + urow];
 }

@@ -469,11 +469,11 @@ int gb_bench_sweep(gb_ctx* ctx, int level, int precision, int reps,
  * The reference aborts on CUDA errors (cuda/check_cuda.h:28-67); this library
  * returns codes. gb_set_wait_limit bounds every device-side wait (the grid
  * barriers of the multi-CTA cycle, GB_MID=1; the dependency waits of the block
- * ILU's cluster; the exchange of the coarsest level's sweeps) to wait_ns
- * nanoseconds (default 1 s): a wait that runs out sets an error flag, the kernel
- * finishes without waiting further, and the call (after a call that only
- * enqueues: the next solve) returns GB_ETIMEOUT with the context still usable. phantoms > 0 makes every such barrier wait for that many CTAs
- * that do not exist, so that its wait runs out (for tests; 0 in normal use).
+ * ILU's cluster) to wait_ns nanoseconds (default 1 s): a wait that runs out sets
+ * an error flag, the kernel finishes without waiting further, and the call
+ * (after a call that only enqueues: the next solve) returns GB_ETIMEOUT with the
+ * context still usable. phantoms > 0 makes every grid barrier wait for that many
+ * CTAs that do not exist, so that its wait runs out (for tests; 0 in normal use).
  * gb_debug_fail_alloc(k): the k-th device allocation from now on fails as an
  * out-of-memory cudaMalloc does (host-side fault injection for tests of the
  * GB_ENOMEM path; 0 turns it off). */
