@@ -1236,7 +1236,8 @@ constexpr int kIluRowsPerLevel = 32; // a CTA's share of an average level
 template<int B, class T, bool UP>
 __device__ __forceinline__ void
 ilu_cluster_run(const IluPack<T>& A, uint32_t y, int rank, const T* in, T* out, T* u, T omega,
-                bool u_zero, volatile int* give_up, unsigned long long wait_ns)
+                bool u_zero, volatile int* give_up, const volatile int* err,
+                unsigned long long wait_ns)
 {
   using W = IluWord<T>;
   using U = typename W::U;
@@ -1249,19 +1250,21 @@ ilu_cluster_run(const IluPack<T>& A, uint32_t y, int rank, const T* in, T* out, 
   int g = A.gptr[rank] + int(threadIdx.x >> 5);
   if (g >= g1)
     return;
-  // after a round of polls: whether the warp gives up (after wait_ns, or with
-  // another warp of the CTA)
+  // after a round of polls: whether the warp gives up, which it does when one
+  // wait has taken wait_ns, with another warp of the CTA, or with a wait of an
+  // earlier launch that nothing has reported yet; it then waits no more
   unsigned spins = 0;
   unsigned long long t0 = 0;
+  bool ended = __any_sync(kAll, *give_up);
   auto expired = [&]() -> bool {
-    if ((++spins & 1023u) != 0)
-      return false;
+    if (ended || (++spins & 1023u) != 0)
+      return ended;
     const unsigned long long t = global_ns();
     t0 = t0 ? t0 : t;
-    const bool end = __any_sync(kAll, *give_up || t - t0 > wait_ns);
-    if (end)
+    ended = __any_sync(kAll, *give_up || *err || t - t0 > wait_ns);
+    if (ended)
       *give_up = 1;
-    return end;
+    return ended;
   };
   int ni = __ldg(A.row + int64_t(g) * kSlice + lane);
   int n0 = __ldg(A.base + g), n1 = __ldg(A.base + g + 1);
@@ -1319,6 +1322,8 @@ ilu_cluster_run(const IluPack<T>& A, uint32_t y, int rank, const T* in, T* out, 
       auto consume = [&](auto is_far, auto half) {
         constexpr bool kFar = decltype(is_far)::value;
         constexpr int h = decltype(half)::value * H;
+        spins = 0; // a wait of its own
+        t0 = 0;
         // what a row waits for longest is mostly its last entry: that one is
         // polled alone (a load and a vote), then all are read
         while (__any_sync(kAll, W::upper(W::template load<kFar>(at[h + H - 1])) ==
@@ -1429,11 +1434,13 @@ ilu_cluster_run(const IluPack<T>& A, uint32_t y, int rank, const T* in, T* out, 
 // level. Levels whose y exceeds the cluster's shared memory (about 440,000 rows
 // in FP64, twice that in FP32) keep the level launches. Every wait ends: a row
 // waits only for rows of earlier levels, a warp takes its groups in level
-// order, and the CTAs of a cluster run at the same time; bounded all the same.
+// order, and the CTAs of a cluster run at the same time; bounded all the same, by
+// wait_ns for each wait. A warp that gives up goes through its remaining groups
+// without waiting, so every row is stored and every thread reaches the barriers.
 template<int B, class T>
 __global__ void __launch_bounds__(ilu_threads<T>(), 1)
 k_ilu_cluster(IluPack<T> lo, IluPack<T> up, int n, const T* rhs, T* h, T* u, double omega,
-              int u_zero, int* err, unsigned long long wait_ns)
+              int u_zero, int* err, unsigned long long wait_ns, unsigned phantoms)
 {
   extern __shared__ __align__(16) unsigned char ilu_smem[];
   __shared__ int give_up;
@@ -1451,17 +1458,21 @@ k_ilu_cluster(IluPack<T> lo, IluPack<T> up, int n, const T* rhs, T* h, T* u, dou
   };
   if (threadIdx.x == 0)
     give_up = 0;
-  if (threadIdx.x < B) // what the entries before a row's first one read
-    W::store(y + uint32_t(lo.chunk * B + threadIdx.x) * uint32_t(sizeof(T)), 0);
+  // what the entries before a row's first one read; with phantoms (a test) it
+  // never comes
+  if (threadIdx.x < B)
+    W::store(y + uint32_t(lo.chunk * B + threadIdx.x) * uint32_t(sizeof(T)),
+             phantoms ? W::kMark : 0);
   GB_PDL_ENTRY();
   mark(lo);
   cluster_barrier();
-  ilu_cluster_run<B, T, false>(lo, y, int(rank), rhs, h, nullptr, T(0), false, &give_up, wait_ns);
+  ilu_cluster_run<B, T, false>(lo, y, int(rank), rhs, h, nullptr, T(0), false, &give_up, err,
+                               wait_ns);
   cluster_barrier();
   mark(up);
   cluster_barrier();
   ilu_cluster_run<B, T, true>(up, y, int(rank), h, h, u, static_cast<T>(omega), u_zero != 0,
-                              &give_up, wait_ns);
+                              &give_up, err, wait_ns);
   cluster_barrier(); // no CTA leaves while another reads its part of y
   if (threadIdx.x == 0 && give_up)
     atomicExch(err, 1);

@@ -333,7 +333,7 @@ void Emit<T>::ilu_cluster(int l, const T* rhs, T* h, T* u, bool u_zero)
                                  int(kIluClusterBytes + 32)));
     launch_cluster(c, kern, L.ilu_ctas, ilu_threads<T>(), int(smem), ilu_pack_of<T>(L, 0),
                    ilu_pack_of<T>(L, 1), (int)L.n, rhs, h, u, c.params.omega, int(u_zero),
-                   c.miderr.p, c.wait_ns);
+                   c.miderr.p, c.wait_ns, c.barrier_phantoms);
   };
   switch (L.B) {
     case 1: run(k_ilu_cluster<1, T>); break;

@@ -473,7 +473,8 @@ int gb_bench_sweep(gb_ctx* ctx, int level, int precision, int reps,
  * an error flag, the kernel finishes without waiting further, and the call
  * (after a call that only enqueues: the next solve) returns GB_ETIMEOUT with the
  * context still usable. phantoms > 0 makes every grid barrier wait for that many
- * CTAs that do not exist, so that its wait runs out (for tests; 0 in normal use).
+ * CTAs that do not exist, and every dependency wait for a value that never comes,
+ * so that it runs out (for tests; 0 in normal use).
  * gb_debug_fail_alloc(k): the k-th device allocation from now on fails as an
  * out-of-memory cudaMalloc does (host-side fault injection for tests of the
  * GB_ENOMEM path; 0 turns it off). */
