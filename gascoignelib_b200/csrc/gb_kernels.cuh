@@ -2019,10 +2019,11 @@ cluster_barrier()
 // ends the sweep. Measured on 16 CTAs, 9 sweeps with events around the launch:
 // 29 us for 1,331 Q2 rows in FP32, 38 us in FP64, 31 us for 3,375 Q1 rows in
 // FP64; 8 CTAs 6 to 8 us more. (Counting every value on the receiver's mbarrier
-// in place of the barrier: 27, 37 and 29 us, but nothing then tells a CTA that is
+// in place of the barrier: 27, 37 and 25 us, but nothing then tells a CTA that is
 // ahead that another CTA's threads have read their partial sums, and a wait that
-// ran out would leave values under way.) Solves against a launch per sweep: 80^3
-// Q2 cells 51.1 -> 46.5 ms, 40^3 Q2 cells with a refined ball 51.9 -> 46.9 ms.
+// ran out would leave values under way.) Solves with a launch per sweep and with
+// this: 80^3 Q2 cells 41.8 and 41.6 ms, 40^3 Q2 cells with a refined ball 43.5
+// and 43.1 ms, 56^3 Q1 cells (left) 1.76 and 1.74 ms.
 // Why nothing is overwritten while it is read: a sweep's last reads of `part`
 // and of the old copy of x come before its cluster barrier, for every thread of
 // every CTA, and the next sweep, which is the next to write `part` and the old
