@@ -105,8 +105,9 @@ int
 gb_ctx_synchronize(gb_ctx* ctx)
 {
   GB_API_BEGIN
+  wait_flag_enqueue(*ctx);
   GB_CUDA(cudaStreamSynchronize(ctx->stream));
-  throw_if_wait_ended(*ctx);
+  wait_flag_check(*ctx);
   GB_API_END
 }
 
@@ -432,8 +433,9 @@ gb_vec_download(gb_ctx* ctx, int lvl, int id, double* host, int64_t len)
   GB_REQUIRE(host && len == ctx->L[lvl].ndof(), GB_EINVAL, "length differs from level size");
   GB_CUDA(cudaMemcpyAsync(host, d, len * sizeof(double), cudaMemcpyDeviceToHost,
                           ctx->stream));
+  wait_flag_enqueue(*ctx);
   GB_CUDA(cudaStreamSynchronize(ctx->stream));
-  throw_if_wait_ended(*ctx);
+  wait_flag_check(*ctx);
   GB_API_END
 }
 

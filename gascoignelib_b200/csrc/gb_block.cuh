@@ -1475,7 +1475,7 @@ k_ilu_cluster(IluPack<T> lo, IluPack<T> up, int n, const T* rhs, T* h, T* u, dou
                               &give_up, err, wait_ns);
   cluster_barrier(); // no CTA leaves while another reads its part of y
   if (threadIdx.x == 0 && give_up)
-    atomicExch(err, 1);
+    atomicCAS(err, 0, kWaitIlu);
 }
 
 // u = (u_zero ? 0 : u) + omega h (StdSolver::Add after the ILU solve, unfused)

@@ -746,7 +746,8 @@ bool direct_on(const Context& c);
 void ensure_vanka(Context& c, Level& L);
 void ensure_ilu(Context& c, Level& L);
 void ensure_wait_flag(Context& c);
-void throw_if_wait_ended(Context& c);
+void wait_flag_enqueue(Context& c);
+void wait_flag_check(Context& c);
 // whether k_ilu_cluster runs level L's substitutions on values of T
 template<class T>
 inline bool

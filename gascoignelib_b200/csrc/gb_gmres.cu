@@ -97,10 +97,7 @@ fill_info_enqueue(Context& c, const double* x_for_residual, const double* b)
   auto* st = c.h_status;
   GB_CUDA(cudaMemcpyAsync(&st->info, &c.G.p->info, sizeof(CGInfoDev), cudaMemcpyDeviceToHost,
                           c.stream));
-  st->mid_err = 0;
-  if (c.miderr.p)
-    GB_CUDA(cudaMemcpyAsync(&st->mid_err, c.miderr.p, sizeof(int), cudaMemcpyDeviceToHost,
-                            c.stream));
+  wait_flag_enqueue(c);
   // true residual ||b - A x|| and ||b|| (FP64)
   const int fl = c.nlevels - 1;
   Level& L = c.L[fl];
@@ -117,10 +114,6 @@ void
 fill_info_finish(Context& c, gb_solve_info* info)
 {
   auto* st = c.h_status;
-  if (st->mid_err) {
-    GB_CUDA(cudaMemsetAsync(c.miderr.p, 0, sizeof(int), c.stream));
-    throw Error{ GB_ETIMEOUT, "a grid barrier of the multi-CTA cycle gave up waiting" };
-  }
   info->iterations = st->info.iteration;
   info->status = st->info.status;
   info->firstresidual = st->info.firstresidual;
@@ -135,6 +128,7 @@ fill_info(Context& c, gb_solve_info* info, double* x_for_residual, const double*
 {
   fill_info_enqueue(c, x_for_residual, b);
   GB_CUDA(cudaStreamSynchronize(c.stream));
+  wait_flag_check(c);
   fill_info_finish(c, info);
 }
 
@@ -205,7 +199,9 @@ gmres_left_mgs(Context& c, double* x, const double* b, gb_solve_info* info)
   }
   final_filter(c, x);
   GB_CUDA(cudaEventRecord(c.ev1, c.stream));
-  GB_CUDA(cudaEventSynchronize(c.ev1));
+  wait_flag_enqueue(c);
+  GB_CUDA(cudaStreamSynchronize(c.stream));
+  wait_flag_check(c);
   float ms = 0;
   GB_CUDA(cudaEventElapsedTime(&ms, c.ev0, c.ev1));
   if (info) {
@@ -307,7 +303,9 @@ gmres_flexible(Context& c, double* x, const double* b, int prec, gb_solve_info* 
   }
   final_filter(c, x);
   GB_CUDA(cudaEventRecord(c.ev1, c.stream));
-  GB_CUDA(cudaEventSynchronize(c.ev1));
+  wait_flag_enqueue(c);
+  GB_CUDA(cudaStreamSynchronize(c.stream));
+  wait_flag_check(c);
   float ms = 0;
   GB_CUDA(cudaEventElapsedTime(&ms, c.ev0, c.ev1));
   if (info) {
@@ -624,7 +622,10 @@ fgmres_graph(Context& c, double* x, const double* b, int prec, gb_solve_info* in
                           cudaMemcpyDeviceToHost, c.stream));
   if (info)
     fill_info_enqueue(c, c.xg.p, c.bg.p);
+  else
+    wait_flag_enqueue(c);
   GB_CUDA(cudaStreamSynchronize(c.stream));
+  wait_flag_check(c);
   float ms = 0;
   GB_CUDA(cudaEventElapsedTime(&ms, c.ev0, c.ev1));
   const int total = st->total, restarts = st->restarts, conv = st->converged;
@@ -813,7 +814,10 @@ gmres_left(Context& c, double* x, const double* b, gb_solve_info* info)
   GB_CUDA(cudaMemcpyAsync(st + 3, &c.G.p->j, sizeof(int), cudaMemcpyDeviceToHost, c.stream));
   if (info)
     fill_info_enqueue(c, c.xg.p, c.bg.p);
+  else
+    wait_flag_enqueue(c);
   GB_CUDA(cudaStreamSynchronize(c.stream));
+  wait_flag_check(c);
   int64_t kernels = c.launches - l0;
   if (graph) {
     const int64_t in_graph = LG.setup_k + int64_t(st[3]) * LG.inner_k;

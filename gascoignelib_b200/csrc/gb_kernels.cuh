@@ -1903,6 +1903,10 @@ k_coarse_cycle(const CoarseOp* __restrict__ ops, int nops,
 // the host reports GB_ETIMEOUT and clears the flag).
 constexpr int kMidThreads = 256;
 
+// what the error flag says: which kind of wait ran out (0: none)
+constexpr int kWaitGrid = 1; // a grid barrier of the multi-CTA cycle
+constexpr int kWaitIlu = 2;  // a dependency wait of the block ILU's cluster
+
 __device__ __forceinline__ unsigned long long
 global_ns()
 {
@@ -1926,7 +1930,7 @@ mid_barrier(unsigned* bar, unsigned target, int* err, unsigned long long wait_ns
       if (v >= target)
         break;
       if (*reinterpret_cast<volatile int*>(err) || global_ns() - t0 > wait_ns) {
-        atomicExch(err, 1);
+        atomicCAS(err, 0, kWaitGrid);
         break;
       }
     }

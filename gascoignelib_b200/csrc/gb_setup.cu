@@ -782,20 +782,31 @@ ensure_wait_flag(Context& c)
   GB_CUDA(cudaMemsetAsync(c.miderr.p, 0, sizeof(int), c.stream));
 }
 
-// After a synchronisation: reports (and clears) a wait that gave up in a call
-// that returned before its kernels had run. Only the substitution clusters
-// wait in such calls.
+// Copies the flag to the host with the stream's other work, for wait_flag_check
+// after the synchronisation that the caller does anyway. Only the multi-CTA cycle
+// and the substitution cluster have waits that can run out.
 void
-throw_if_wait_ended(Context& c)
+wait_flag_enqueue(Context& c)
 {
-  if (!c.ilu_max_ctas || !c.miderr.p)
-    return;
-  int err = 0;
-  GB_CUDA(cudaMemcpy(&err, c.miderr.p, sizeof(int), cudaMemcpyDeviceToHost));
+  c.h_status->mid_err = 0;
+  if (c.miderr.p && (c.mid_on || c.ilu_max_ctas))
+    GB_CUDA(cudaMemcpyAsync(&c.h_status->mid_err, c.miderr.p, sizeof(int),
+                            cudaMemcpyDeviceToHost, c.stream));
+}
+
+// Reports (and clears) a wait that gave up in this call or in one before it that
+// only enqueued its kernels.
+void
+wait_flag_check(Context& c)
+{
+  const int err = c.h_status->mid_err;
   if (!err)
     return;
+  c.h_status->mid_err = 0;
   GB_CUDA(cudaMemsetAsync(c.miderr.p, 0, sizeof(int), c.stream));
-  throw Error{ GB_ETIMEOUT, "a dependency wait of the block ILU gave up waiting" };
+  throw Error{ GB_ETIMEOUT, err == kWaitIlu
+                              ? "a dependency wait of the block ILU gave up waiting"
+                              : "a grid barrier of the multi-CTA cycle gave up waiting" };
 }
 
 // CTAs of the largest cluster (16, a size that is not portable, or 8) the

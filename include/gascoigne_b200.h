@@ -470,9 +470,9 @@ int gb_bench_sweep(gb_ctx* ctx, int level, int precision, int reps,
  * returns codes. gb_set_wait_limit bounds every device-side wait (the grid
  * barriers of the multi-CTA cycle, GB_MID=1; the dependency waits of the block
  * ILU's cluster) to wait_ns nanoseconds (default 1 s): a wait that runs out sets
- * an error flag, the kernel finishes without waiting further, and the call
- * (after a call that only enqueues: the next solve) returns GB_ETIMEOUT with the
- * context still usable. phantoms > 0 makes every grid barrier wait for that many
+ * an error flag, the kernel finishes without waiting further, and the call (after
+ * a call that only enqueues: the next solve, gb_vec_download or
+ * gb_ctx_synchronize) returns GB_ETIMEOUT with the context still usable. phantoms > 0 makes every grid barrier wait for that many
  * CTAs that do not exist, and every dependency wait for a value that never comes,
  * so that it runs out (for tests; 0 in normal use).
  * gb_debug_fail_alloc(k): the k-th device allocation from now on fails as an
