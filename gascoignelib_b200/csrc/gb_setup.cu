@@ -795,7 +795,9 @@ wait_flag_enqueue(Context& c)
 }
 
 // Reports (and clears) a wait that gave up in this call or in one before it that
-// only enqueued its kernels.
+// only enqueued its kernels. What the context may have formed with such kernels
+// (the coarse levels' maps, and the solver graphs that launch them) is formed
+// again by the next call.
 void
 wait_flag_check(Context& c)
 {
@@ -803,6 +805,8 @@ wait_flag_check(Context& c)
   if (!err)
     return;
   c.h_status->mid_err = 0;
+  c.work_ready = false;
+  c.version++;
   GB_CUDA(cudaMemsetAsync(c.miderr.p, 0, sizeof(int), c.stream));
   throw Error{ GB_ETIMEOUT, err == kWaitIlu
                               ? "a dependency wait of the block ILU gave up waiting"
