@@ -2,6 +2,7 @@
 // systems), the pressure filter, the Vanka smoother and the block ILU.
 // Included by gb_context.cuh after gb_kernels.cuh.
 #pragma once
+#include "gb_ilu_plan.cuh"
 #include "gb_kernels.cuh"
 #include <type_traits>
 
@@ -1092,8 +1093,6 @@ struct IluPack
 };
 
 constexpr int kIluPush = 2;
-constexpr int kIluOwnerShift = 24;
-constexpr int kIluPlaceMask = (1 << kIluOwnerShift) - 1;
 
 // The "not yet computed" mark of a word of y: all bits set, a NaN. It is told
 // by the upper 32 bits, and a computed value with such bits is stored as
@@ -1225,8 +1224,6 @@ ilu_threads()
 {
   return sizeof(T) == 4 ? 768 : 512;
 }
-constexpr size_t kIluClusterBytes = 216 * 1024; // of y in a CTA's shared memory
-constexpr int kIluRowsPerLevel = 32; // a CTA's share of an average level
 
 // One direction of k_ilu_cluster: this CTA's groups, warp by warp in level
 // order. in: the rows' right-hand side; out: the result in global memory. All

@@ -297,8 +297,10 @@ struct Level
   };
   std::vector<IluSeg> ilu_lseg, ilu_useg;
   // the packed factors of the cluster substitution (k_ilu_cluster), forward 0
-  // and backward 1; ctas 0: the level's rows do not fit a cluster
+  // and backward 1 (IluPlan: ctas 0, the level does not run in a cluster; FP64
+  // values only with ilu_fp64)
   int ilu_ctas = 0, ilu_chunk = 0, ilu_groups[2] = { 0, 0 };
+  bool ilu_fp64 = false;
   DeviceArray<int> ilu_gptr[2], ilu_grow[2], ilu_gbase[2], ilu_gcol[2];
   DeviceArray<int> ilu_push[2], ilu_gofs[2], ilu_ghost[2]; // copies of other CTAs' rows
   int ilu_places = 0; // of y in a CTA's shared memory, in rows
@@ -748,12 +750,13 @@ void ensure_ilu(Context& c, Level& L);
 void ensure_wait_flag(Context& c);
 void wait_flag_enqueue(Context& c);
 void wait_flag_check(Context& c);
-// whether k_ilu_cluster runs level L's substitutions on values of T
+// whether k_ilu_cluster runs level L's substitutions on values of T: where
+// ilu_groups made the packed factors for them
 template<class T>
 inline bool
-ilu_in_cluster(const Context& c, const Level& L)
+ilu_in_cluster(const Level& L)
 {
-  return L.ilu_ctas > 0 && size_t(L.ilu_places) * L.B * sizeof(T) <= kIluClusterBytes + 32;
+  return L.ilu_ctas > 0 && (sizeof(T) == 4 || L.ilu_fp64);
 }
 void ensure_work(Context& c);
 

@@ -330,7 +330,7 @@ void Emit<T>::ilu_cluster(int l, const T* rhs, T* h, T* u, bool u_zero)
     const size_t smem = size_t(L.ilu_places) * L.B * sizeof(T);
     GB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
     GB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 int(kIluClusterBytes + 32)));
+                                 int(kIluClusterBytes + kIluZeroBytes)));
     launch_cluster(c, kern, L.ilu_ctas, ilu_threads<T>(), int(smem), ilu_pack_of<T>(L, 0),
                    ilu_pack_of<T>(L, 1), (int)L.n, rhs, h, u, c.params.omega, int(u_zero),
                    c.miderr.p, c.wait_ns, c.barrier_phantoms);
@@ -549,7 +549,7 @@ smooth(Emit<T>& E, int l, int niter, T*& u, T*& tmp, const T* b, bool& u_zero)
     if (c.params.smoother == 2) {
       // linear_smooth ilu: h = y - A u (filtered), the ILU solve of h in
       // place, u += omega h, SubtractMean(u) (StdSolver::smooth)
-      const bool cluster = ilu_in_cluster<T>(c, L);
+      const bool cluster = ilu_in_cluster<T>(L);
       const T* h = tmp;
       if (!u_zero)
         E.resid(l, u, tmp, b);

@@ -845,9 +845,7 @@ max_ctas(K* kern, int threads, size_t smem)
 
 // How the level's rows are shared out among the CTAs of k_ilu_cluster, and the
 // groups of each (once per matrix structure). lev: the rows' dependency levels
-// per direction. The cluster is the smallest power of two whose shared memory
-// holds y and in which a level of average width gives each CTA at most two
-// groups.
+// per direction.
 static void
 ilu_groups(Context& c, Level& L, const std::vector<int> (&lev)[2], const int (&nlev)[2],
            const std::vector<int>& ptr, const std::vector<int>& col,
@@ -855,21 +853,15 @@ ilu_groups(Context& c, Level& L, const std::vector<int> (&lev)[2], const int (&n
 {
   L.ilu_ctas = 0;
   const int64_t n = L.n;
-  if (!c.ilu_cluster || (n + 1) * L.B >= (int64_t(1) << kIluOwnerShift))
+  if (!c.ilu_cluster)
     return;
   if (!c.ilu_max_ctas)
-    c.ilu_max_ctas = max_ctas(k_ilu_cluster<1, double>, ilu_threads<double>(), kIluClusterBytes + 32);
-  const int most = c.ilu_max_ctas;
-  auto bytes = [&](int ctas, size_t size) { return size_t((n + ctas - 1) / ctas) * L.B * size; };
-  const size_t size = bytes(most, 8) <= kIluClusterBytes ? 8 : 4;
-  if (bytes(most, size) > kIluClusterBytes)
+    c.ilu_max_ctas = max_ctas(k_ilu_cluster<1, double>, ilu_threads<double>(),
+                              kIluClusterBytes + kIluZeroBytes);
+  const IluPlan P = ilu_plan(n, L.B, nlev[0], c.ilu_max_ctas);
+  if (!P.ctas)
     return;
-  int ctas = 1;
-  while (ctas < most &&
-         (bytes(ctas, size) > kIluClusterBytes ||
-          n > int64_t(ctas) * nlev[0] * kIluRowsPerLevel))
-    ctas *= 2;
-  const int chunk = static_cast<int>((n + ctas - 1) / ctas), half = ilu_half(L.B);
+  const int ctas = P.ctas, chunk = P.chunk, half = ilu_half(L.B);
   // the rows of other CTAs that each CTA uses, and where each row is used
   std::vector<int> gofs[2], ghost[2], push[2];
   int copies = 0;
@@ -901,8 +893,7 @@ ilu_groups(Context& c, Level& L, const std::vector<int> (&lev)[2], const int (&n
     }
   }
   // not where a row goes to many CTAs or the copies do not fit
-  if (!pushed || size_t(chunk + 1 + copies) * L.B * size > kIluClusterBytes ||
-      int64_t(chunk + 1 + copies) * L.B >= (int64_t(1) << kIluOwnerShift)) {
+  if (!pushed || !ilu_copies_fit(P, L.B, copies)) {
     copies = 0;
     pushed = false;
     for (int dir = 0; dir < 2; ++dir) {
@@ -971,12 +962,10 @@ ilu_groups(Context& c, Level& L, const std::vector<int> (&lev)[2], const int (&n
       L.ilu_push[dir].release();
     }
     GB_CUDA(L.ilu_gval32[dir].alloc(std::max<size_t>(cols * B2, 1)));
-    if (size == 8)
-      GB_CUDA(L.ilu_gval64[dir].alloc(std::max<size_t>(cols * B2, 1)));
+    GB_CUDA(L.ilu_gval64[dir].alloc(P.fp64 ? std::max<size_t>(cols * B2, 1) : 0));
     if (dir == 1) {
       GB_CUDA(L.ilu_gdinv32.alloc(row.size() * B2));
-      if (size == 8)
-        GB_CUDA(L.ilu_gdinv64.alloc(row.size() * B2));
+      GB_CUDA(L.ilu_gdinv64.alloc(P.fp64 ? row.size() * B2 : 0));
     }
     GB_CUDA(h2d(c.stream, L.ilu_gptr[dir].p, gptr.data(), gptr.size() * sizeof(int)));
     GB_CUDA(h2d(c.stream, L.ilu_grow[dir].p, row.data(), row.size() * sizeof(int)));
@@ -984,6 +973,7 @@ ilu_groups(Context& c, Level& L, const std::vector<int> (&lev)[2], const int (&n
   }
   L.ilu_chunk = chunk;
   L.ilu_ctas = ctas;
+  L.ilu_fp64 = P.fp64;
 }
 
 // The factors into the packed layout of k_ilu_cluster.
@@ -1007,7 +997,7 @@ ilu_pack(Context& c, Level& L)
       pack(k_ilu_pack<float, true>, col, L.ilu_gval32[dir].p, L.ilu_gdinv32.p);
     else
       pack(k_ilu_pack<float, false>, col, L.ilu_gval32[dir].p, L.ilu_gdinv32.p);
-    if (ilu_in_cluster<double>(c, L)) {
+    if (ilu_in_cluster<double>(L)) {
       if (dir)
         pack(k_ilu_pack<double, true>, (int*)nullptr, L.ilu_gval64[dir].p, L.ilu_gdinv64.p);
       else
