@@ -1429,7 +1429,8 @@ ilu_cluster_run(const IluPack<T>& A, uint32_t y, int rank, const T* in, T* out, 
 // threads 18.8 / 16.7 ms for the solve. Rows of an average level per CTA
 // (kIluRowsPerLevel): 64 / 32 / 16 measured 213 / 183 / 180 us on the 33^3
 // level. Levels whose y exceeds the cluster's shared memory (about 440,000 rows
-// in FP64, twice that in FP32) keep the level launches. Every wait ends: a row
+// in FP64, twice that in FP32), and chains whose packed factors would be mostly
+// padding, keep the level launches (gb_ilu_plan.cuh). Every wait ends: a row
 // waits only for rows of earlier levels, a warp takes its groups in level
 // order, and the CTAs of a cluster run at the same time; bounded all the same, by
 // wait_ns for each wait. A warp that gives up goes through its remaining groups

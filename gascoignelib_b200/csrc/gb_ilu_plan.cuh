@@ -56,4 +56,21 @@ ilu_copies_fit(const IluPlan& P, int B, int64_t copies)
          places < (int64_t(1) << kIluOwnerShift);
 }
 
+// Whether the packed factors are worth their memory: `slots` places for a block
+// in both directions together, padding included, for `entries` blocks of the
+// factors. Every (CTA, level) pair takes whole groups of 32 rows, and a row whole
+// chunks of entries: 2 to 3 slots per entry on 3D meshes, up to about 10 on long
+// narrow 2D ones, but 170 for a chain of rows that depend on each other one by
+// one, which at the largest size that fits would be 3.6 GB for 21 MB of factors.
+// Such levels keep the level launches, once the packed form passes 64 MB.
+constexpr int64_t kIluPackBytes = int64_t(64) << 20;
+constexpr int kIluPackRatio = 16;
+inline bool
+ilu_padding_ok(const IluPlan& P, int B, int64_t slots, int64_t entries)
+{
+  const int64_t B2 = int64_t(B) * B;
+  const int64_t packed = slots * (4 + B2 * (P.fp64 ? 12 : 4)); // column, values
+  return packed <= std::max(kIluPackBytes, kIluPackRatio * entries * (4 + B2 * 12));
+}
+
 } // namespace gb

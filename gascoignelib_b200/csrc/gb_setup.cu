@@ -901,7 +901,7 @@ ilu_groups(Context& c, Level& L, const std::vector<int> (&lev)[2], const int (&n
       ghost[dir].clear();
     }
   }
-  L.ilu_places = chunk + 1 + copies;
+  std::vector<int> gptr[2], row[2], base[2];
   for (int dir = 0; dir < 2; ++dir) {
     // rows sorted by (owner, level), ascending within: a counting sort
     const int nl = nlev[dir];
@@ -913,7 +913,8 @@ ilu_groups(Context& c, Level& L, const std::vector<int> (&lev)[2], const int (&n
     at.assign(off.begin(), off.end() - 1);
     for (int64_t i = 0; i < n; ++i)
       order[at[size_t(i / chunk) * nl + lev[dir][i]]++] = static_cast<int>(i);
-    std::vector<int> gptr(ctas + 1, 0), row, base(1, 0);
+    gptr[dir].assign(ctas + 1, 0);
+    base[dir].assign(1, 0);
     for (int r = 0; r < ctas; ++r) {
       for (int q = 0; q < nl; ++q) {
         const int k1 = off[size_t(r) * nl + q + 1];
@@ -922,7 +923,7 @@ ilu_groups(Context& c, Level& L, const std::vector<int> (&lev)[2], const int (&n
           bool far = false; // an entry in another CTA's rows
           for (int l = 0; l < kSlice; ++l) {
             const int i = k + l < k1 ? order[k + l] : -1;
-            row.push_back(i);
+            row[dir].push_back(i);
             if (i < 0)
               continue;
             const int b = dir ? diag[i] + 1 : ptr[i], e = dir ? ptr[i + 1] : diag[i];
@@ -930,19 +931,25 @@ ilu_groups(Context& c, Level& L, const std::vector<int> (&lev)[2], const int (&n
             if (e > b) // ascending columns: the first and the last tell
               far = far || (!pushed && (col[b] / chunk != r || col[e - 1] / chunk != r));
           }
-          GB_REQUIRE(int64_t(base.back() >> 1) + w < (int64_t(1) << 30), GB_EINVAL,
-                     "ILU groups too large");
-          base.back() |= far ? 1 : 0;
-          base.push_back(((base.back() >> 1) + w) << 1);
+          if (int64_t(base[dir].back() >> 1) + w >= (int64_t(1) << 30))
+            return; // beyond the groups' numbering
+          base[dir].back() |= far ? 1 : 0;
+          base[dir].push_back(((base[dir].back() >> 1) + w) << 1);
         }
       }
-      gptr[r + 1] = static_cast<int>(base.size()) - 1;
+      gptr[dir][r + 1] = static_cast<int>(base[dir].size()) - 1;
     }
-    const size_t cols = size_t(base.back() >> 1) * kSlice, B2 = size_t(L.B) * L.B;
-    L.ilu_groups[dir] = static_cast<int>(base.size()) - 1;
-    GB_CUDA(L.ilu_gptr[dir].alloc(gptr.size()));
-    GB_CUDA(L.ilu_grow[dir].alloc(row.size()));
-    GB_CUDA(L.ilu_gbase[dir].alloc(base.size()));
+  }
+  if (!ilu_padding_ok(P, L.B, (int64_t(base[0].back() >> 1) + (base[1].back() >> 1)) * kSlice,
+                      ptr[n]))
+    return;
+  L.ilu_places = chunk + 1 + copies;
+  for (int dir = 0; dir < 2; ++dir) {
+    const size_t cols = size_t(base[dir].back() >> 1) * kSlice, B2 = size_t(L.B) * L.B;
+    L.ilu_groups[dir] = static_cast<int>(base[dir].size()) - 1;
+    GB_CUDA(L.ilu_gptr[dir].alloc(gptr[dir].size()));
+    GB_CUDA(L.ilu_grow[dir].alloc(row[dir].size()));
+    GB_CUDA(L.ilu_gbase[dir].alloc(base[dir].size()));
     GB_CUDA(L.ilu_gcol[dir].alloc(std::max<size_t>(cols, 1)));
     GB_CUDA(L.ilu_gofs[dir].alloc(gofs[dir].size()));
     GB_CUDA(L.ilu_ghost[dir].alloc(std::max<size_t>(ghost[dir].size(), 1)));
@@ -951,11 +958,11 @@ ilu_groups(Context& c, Level& L, const std::vector<int> (&lev)[2], const int (&n
       GB_CUDA(h2d(c.stream, L.ilu_ghost[dir].p, ghost[dir].data(),
                   ghost[dir].size() * sizeof(int)));
     if (pushed) { // per slot, in the groups' order
-      std::vector<int> to(row.size() * kIluPush, -1);
-      for (size_t k = 0; k < row.size(); ++k)
-        for (int q = 0; q < kIluPush && row[k] >= 0; ++q)
+      std::vector<int> to(row[dir].size() * kIluPush, -1);
+      for (size_t k = 0; k < row[dir].size(); ++k)
+        for (int q = 0; q < kIluPush && row[dir][k] >= 0; ++q)
           to[(k / kSlice * kIluPush + q) * kSlice + k % kSlice] =
-            push[dir][size_t(row[k]) * kIluPush + q];
+            push[dir][size_t(row[dir][k]) * kIluPush + q];
       GB_CUDA(L.ilu_push[dir].alloc(to.size()));
       GB_CUDA(h2d(c.stream, L.ilu_push[dir].p, to.data(), to.size() * sizeof(int)));
     } else {
@@ -964,12 +971,12 @@ ilu_groups(Context& c, Level& L, const std::vector<int> (&lev)[2], const int (&n
     GB_CUDA(L.ilu_gval32[dir].alloc(std::max<size_t>(cols * B2, 1)));
     GB_CUDA(L.ilu_gval64[dir].alloc(P.fp64 ? std::max<size_t>(cols * B2, 1) : 0));
     if (dir == 1) {
-      GB_CUDA(L.ilu_gdinv32.alloc(row.size() * B2));
-      GB_CUDA(L.ilu_gdinv64.alloc(P.fp64 ? row.size() * B2 : 0));
+      GB_CUDA(L.ilu_gdinv32.alloc(row[dir].size() * B2));
+      GB_CUDA(L.ilu_gdinv64.alloc(P.fp64 ? row[dir].size() * B2 : 0));
     }
-    GB_CUDA(h2d(c.stream, L.ilu_gptr[dir].p, gptr.data(), gptr.size() * sizeof(int)));
-    GB_CUDA(h2d(c.stream, L.ilu_grow[dir].p, row.data(), row.size() * sizeof(int)));
-    GB_CUDA(h2d(c.stream, L.ilu_gbase[dir].p, base.data(), base.size() * sizeof(int)));
+    GB_CUDA(h2d(c.stream, L.ilu_gptr[dir].p, gptr[dir].data(), gptr[dir].size() * sizeof(int)));
+    GB_CUDA(h2d(c.stream, L.ilu_grow[dir].p, row[dir].data(), row[dir].size() * sizeof(int)));
+    GB_CUDA(h2d(c.stream, L.ilu_gbase[dir].p, base[dir].data(), base[dir].size() * sizeof(int)));
   }
   L.ilu_chunk = chunk;
   L.ilu_ctas = ctas;

@@ -58,3 +58,33 @@ def test_largest_levels(n, B):
     for a, b in zip(_results(prob, {}), _results(prob, {"GB_ILU_CTA_ROWS": "0"})):
         assert np.isfinite(a).all()
         assert np.array_equal(a, b)
+
+
+def test_a_long_chain_is_not_packed():
+    # 100,000 rows that depend on each other one by one: 5 MB of factors, 820 MB
+    # in groups of 32 rows and chunks of 8 entries
+    import torch
+    n = 100000
+    i = np.arange(n)
+    rows = np.stack([i - 1, i, i + 1], axis=1)
+    keep = (rows >= 0) & (rows < n)
+    ptr = np.concatenate([[0], np.cumsum(keep.sum(axis=1))]).astype(np.int64)
+    diag = (ptr[:-1] + (i > 0)).astype(np.int64)
+    rng = np.random.default_rng(9)
+    val = rng.uniform(-1.0, 1.0, int(ptr[-1]))
+    val[diag] = 4.0
+    level = Level(n=n, B=1, rowptr=ptr, col=rows[keep].astype(np.int64), diag=diag, val=val,
+                  dirichlet=np.array([], dtype=np.int64))
+    prob = Problem(dim=2, levels=[level], transfers=[], rhs=rng.uniform(-1, 1, n))
+    with Context(0) as ctx:
+        ctx.load_problem(prob)
+        ctx.set_params(omega=1.0, smoother="ilu")
+        x, y, h = ctx.vec(), ctx.vec(), ctx.vec()
+        ctx.upload(0, y, prob.rhs)
+        ctx.zero(0, x)
+        free0, _ = torch.cuda.mem_get_info(0)
+        ctx.smooth(0, 1, x, y, h)
+        ctx.residualgmres(0, h, x, y)
+        assert np.abs(ctx.download(0, h)).max() < 1e-13
+        free1, _ = torch.cuda.mem_get_info(0)
+        assert free0 - free1 < 200 << 20

@@ -75,3 +75,41 @@ def _run(tmp_path, source):
 
 def test_plan_at_its_limits(tmp_path):
     _run(tmp_path, SOURCE)
+
+
+PADDING = r"""
+#include "gb_ilu_plan.cuh"
+#include <cstdio>
+using namespace gb;
+
+// slots of n rows with `lower` and `upper` entries each, `per` rows of a level in a
+// CTA, rounded up to groups of 32 rows and chunks of 8 entries
+static int64_t slots(int64_t n, int per, int lower, int upper)
+{
+  const int64_t groups = (n + per - 1) / per * ((per + 31) / 32);
+  return groups * 32 * ((lower + 7) / 8 * 8 + (upper + 7) / 8 * 8);
+}
+
+int main()
+{
+  auto ok = [](int64_t n, int per, int half) {
+    const IluPlan P = ilu_plan(n, 1, int(n / per / 16 + 1), 16);
+    return P.ctas > 0 && ilu_padding_ok(P, 1, slots(n, per, half, half), n * (2 * half + 1));
+  };
+  const bool r[] = {
+    ok(274625, 38, 13),   // 65^3 rows, 27 entries
+    ok(422500, 13, 4),    // 650^2 rows, 9 entries
+    ok(400000, 6, 4),     // 200 x 2000 rows, numbered along the short side
+    ok(4000, 1, 1),       // a short chain
+    !ok(100000, 1, 1),    // a long one
+    !ok(880000, 1, 1),    // and the longest that fits, in FP32
+  };
+  for (size_t k = 0; k < sizeof r; ++k)
+    if (!r[k]) { printf("rule %zu\n", k); return 1; }
+  return 0;
+}
+"""
+
+
+def test_padding_rule(tmp_path):
+    _run(tmp_path, PADDING)
