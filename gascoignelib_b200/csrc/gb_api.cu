@@ -56,6 +56,8 @@ gb_ctx_create(gb_ctx** out, int device)
     GB_CUDA(ctx->scal.alloc(16));
     GB_CUDA(cudaMallocHost(&ctx->h_flags, 16 * sizeof(int)));
     GB_CUDA(cudaMallocHost(&ctx->h_status, sizeof(gb_ctx::SolveStatus)));
+    GB_CUDA(cudaMallocHost(&ctx->h_upload, gb_ctx::kUploadBytes));
+    GB_CUDA(cudaEventCreateWithFlags(&ctx->ev_upload, cudaEventDisableTiming));
     GB_CUDA(cudaEventCreate(&ctx->evh0));
     GB_CUDA(cudaEventCreate(&ctx->evh1));
   } catch (const gb::Error& e) {
@@ -80,6 +82,10 @@ gb_ctx_destroy(gb_ctx* ctx)
     cudaFreeHost(ctx->h_flags);
   if (ctx->h_status)
     cudaFreeHost(ctx->h_status);
+  if (ctx->h_upload)
+    cudaFreeHost(ctx->h_upload);
+  if (ctx->ev_upload)
+    cudaEventDestroy(ctx->ev_upload);
   if (ctx->evh0)
     cudaEventDestroy(ctx->evh0);
   if (ctx->evh1)
@@ -410,16 +416,27 @@ gb_vec_upload(gb_ctx* ctx, int lvl, int id, const double* host, int64_t len)
   GB_API_BEGIN
   double* d = vec(*ctx, lvl, id);
   GB_REQUIRE(host && len == ctx->L[lvl].ndof(), GB_EINVAL, "length differs from level size");
-  GB_CUDA(cudaMemcpyAsync(d, host, len * sizeof(double), cudaMemcpyHostToDevice,
-                          ctx->stream));
-  // A copy from pageable memory returns when the source has been read (it is
-  // staged); the rest of it is ordered by the stream. Any other source (pinned,
-  // managed) may still be read after the call returns: wait for it. A cycle of a
-  // host Krylov loop on a small problem spent 6 of 54 us in this wait.
+  const size_t bytes = len * sizeof(double);
+  // The source may change when the call has returned. A small pageable one is
+  // copied into the context's own pinned buffer first, and the stream reads it from
+  // there: a cycle of a host Krylov loop on a small problem spent 6 of 54 us waiting
+  // for its upload. (Not left to the runtime's staging of pageable memory: where
+  // the device reads such memory itself, it need not stage it.) Others, and sources
+  // that the stream's own work may write (pinned, managed), are waited for.
   cudaPointerAttributes at{};
-  if (cudaPointerGetAttributes(&at, host) != cudaSuccess ||
-      at.type != cudaMemoryTypeUnregistered) {
-    cudaGetLastError();
+  bool pageable = true;
+  if (cudaPointerGetAttributes(&at, host) != cudaSuccess) {
+    cudaGetLastError(); // leave no error behind
+    pageable = false;
+  }
+  pageable = pageable && at.type == cudaMemoryTypeUnregistered;
+  if (pageable && bytes <= gb_ctx::kUploadBytes) {
+    GB_CUDA(cudaEventSynchronize(ctx->ev_upload)); // the upload before has been read
+    memcpy(ctx->h_upload, host, bytes);
+    GB_CUDA(cudaMemcpyAsync(d, ctx->h_upload, bytes, cudaMemcpyHostToDevice, ctx->stream));
+    GB_CUDA(cudaEventRecord(ctx->ev_upload, ctx->stream));
+  } else {
+    GB_CUDA(cudaMemcpyAsync(d, host, bytes, cudaMemcpyHostToDevice, ctx->stream));
     GB_CUDA(cudaStreamSynchronize(ctx->stream));
   }
   GB_API_END

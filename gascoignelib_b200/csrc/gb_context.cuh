@@ -401,6 +401,10 @@ struct gb_ctx
   };
   SolveStatus* h_status = nullptr;
   cudaEvent_t evh0 = nullptr, evh1 = nullptr; // gb_solve_host's window
+  // pinned staging of small uploads, and when the stream has read it
+  static constexpr size_t kUploadBytes = size_t(256) << 10;
+  double* h_upload = nullptr;
+  cudaEvent_t ev_upload = nullptr;
   int64_t launches = 0;
   gb::DeviceArray<unsigned char> flush;
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;

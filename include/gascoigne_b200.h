@@ -182,6 +182,7 @@ int gb_level_set_pfilter(gb_ctx* ctx, int level, int comp_mask,
  * StdSolver's vector ops (Solver/stdsolver.cc:685-688,1775-1810). */
 int gb_vec_create(gb_ctx* ctx, int* id);
 int gb_vec_free(gb_ctx* ctx, int id);
+/* host may be changed or freed once the call has returned */
 int gb_vec_upload(gb_ctx* ctx, int level, int id, const double* host,
                   int64_t len);
 int gb_vec_download(gb_ctx* ctx, int level, int id, double* host, int64_t len);
