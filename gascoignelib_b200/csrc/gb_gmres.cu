@@ -782,9 +782,11 @@ gmres_left(Context& c, double* x, const double* b, gb_solve_info* info)
   // A program may solve once per matrix (a Newton step that uploads new values):
   // building the graph (about 2 ms) takes longer than the launches it saves in
   // one solve, so it is built by the second solve with the same levels and keys.
-  // Both ways give the same bits.
-  bool graph = c.use_graph && LG.exec && LG.version == c.version;
-  if (c.use_graph && !graph && LG.seen == c.version) {
+  // Both ways give the same bits. Kernels in a graph are not timed one by one, so
+  // with gb_set_timing every solve launches them.
+  const bool allowed = c.use_graph && !c.ktime;
+  bool graph = allowed && LG.exec && LG.version == c.version;
+  if (allowed && !graph && LG.seen == c.version) {
     build_left_graph(c);
     graph = true;
   }
