@@ -560,9 +560,25 @@ k_vanka_factor(int npatch, int npp, int B, int M, const int* __restrict__ map,
 // Patches of more than 32 unknowns (3D: 108): one CTA of kVankaWide warps per
 // patch, warp q taking the columns j = q, q + kVankaWide, ..; a row's partial
 // sums are added in the warps' order. With a warp per patch the 512 patches of
-// a 17^3 Stokes level were 3.5 warps per SM with 12 loads each in flight: 29 us
-// against 7.4 us for their 48 MB at the copy rate.
+// a 17^3 Stokes level were 3.5 warps per SM with 12 loads each in flight: 27 us
+// against 7.4 us for their 48 MB at the copy rate; 10.7 us in this form.
 constexpr int kVankaWide = 8;
+
+// Taken up to so many patches; with more of them a warp per patch fills the SMs and
+// the two block barriers of a patch are what is left to see. Warp and CTA, us with
+// events around the launch, patches of 27 nodes:
+//   54 unknowns, FP64: 1,000 10.7 10.6; 1,728 10.8 12.9; 13,824 62 111
+//                FP32: 1,000 10.6 8.6; 1,728 10.6 10.7; 13,824 37 62
+//   81 unknowns, FP64: 1,728 33.7 24.9; 2,744 41.4 45.7; 13,824 122 171
+//                FP32: 1,728 13.8 12.8; 2,744 18.8 17.0; 4,096 27.8 33.3
+//  108 unknowns, FP64: 4,096 81.7 74.3; 5,832 99.6 100.9; 13,824 214 222
+//                FP32: 2,744 37.2 36.5; 4,096 44.7 47.4; 13,824 120 134
+template<class T>
+constexpr int
+vanka_wide_patches(int R)
+{
+  return R == 2 ? 1000 : R == 3 ? 2000 : sizeof(T) == 8 ? 5000 : 3000;
+}
 template<int R, class TL, class T>
 __global__ void __launch_bounds__(32 * kVankaWide)
 k_vanka_inv_wide(int npatch, int M, int B, const int* __restrict__ pn,

@@ -70,22 +70,25 @@ void Emit<T>::vanka(int l, const T* h, T* u, bool u_zero, const double* hmean)
     else
       launch(c, k_vanka_inv_ct<9, T, T>, nbp, 32 * kVankaWarps, L.npatch, L.B,
              (const int*)L.vk_pn.p, inv, h, pc, hmean, out);
-  } else switch ((L.vk_M + 31) / 32) {
-    case 1:
-      launch(c, k_vanka_inv<1, T, T>, nbp, 32 * kVankaWarps, L.npatch, L.vk_M, L.B,
-             (const int*)L.vk_pn.p, inv, h, pc, hmean, out);
-      break;
-    case 2:
-      launch(c, k_vanka_inv_wide<2, T, T>, L.npatch, 32 * kVankaWide, L.npatch, L.vk_M, L.B,
-             (const int*)L.vk_pn.p, inv, h, pc, hmean, out);
-      break;
-    case 3:
-      launch(c, k_vanka_inv_wide<3, T, T>, L.npatch, 32 * kVankaWide, L.npatch, L.vk_M, L.B,
-             (const int*)L.vk_pn.p, inv, h, pc, hmean, out);
-      break;
-    default:
-      launch(c, k_vanka_inv_wide<4, T, T>, L.npatch, 32 * kVankaWide, L.npatch, L.vk_M, L.B,
-             (const int*)L.vk_pn.p, inv, h, pc, hmean, out);
+  } else {
+    auto patches = [&](auto rows) { // of 32 unknowns in a patch
+      constexpr int R = decltype(rows)::value;
+      if (L.npatch <= vanka_wide_patches<T>(R))
+        launch(c, k_vanka_inv_wide<R, T, T>, L.npatch, 32 * kVankaWide, L.npatch, L.vk_M, L.B,
+               (const int*)L.vk_pn.p, inv, h, pc, hmean, out);
+      else
+        launch(c, k_vanka_inv<R, T, T>, nbp, 32 * kVankaWarps, L.npatch, L.vk_M, L.B,
+               (const int*)L.vk_pn.p, inv, h, pc, hmean, out);
+    };
+    switch ((L.vk_M + 31) / 32) {
+      case 1:
+        launch(c, k_vanka_inv<1, T, T>, nbp, 32 * kVankaWarps, L.npatch, L.vk_M, L.B,
+               (const int*)L.vk_pn.p, inv, h, pc, hmean, out);
+        break;
+      case 2: patches(std::integral_constant<int, 2>{}); break;
+      case 3: patches(std::integral_constant<int, 3>{}); break;
+      default: patches(std::integral_constant<int, 4>{});
+    }
   }
   const PfArgs pf = weighted_mean_args(L);
   const int nb = blocks_for(L.ndof(), 256);
