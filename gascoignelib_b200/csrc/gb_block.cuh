@@ -130,13 +130,27 @@ bspmv_component(const SellView<TV>& A, const TX* __restrict__ x, int s, int lane
 
 // k_bspmv with a thread per row and component (warp = slice and component): a
 // thread has B of a block's B^2 values to load, and there are B times as many
-// threads. For the levels of at most kBlockSplitRows rows, whose one thread per
-// row leaves most of the GPU idle and is a chain of 27 x B^2 loads. Measured
-// with events around the launch: residual of 17^3 rows, B = 4, FP64 30 -> 15
-// us; of the seven levels below 513^2 rows, B = 3, FP32 about 14 -> 11.8 us
-// each. On the 513^2 level itself the x loads, B times as many, cost more than
-// they gain (the solve 13.9 -> 14.3 ms), so it keeps one thread per row.
-constexpr int64_t kBlockSplitRows = 100000;
+// threads. For small levels (block_split), whose one thread per row leaves most
+// of the GPU idle and is a chain of 27 x B^2 loads. Measured with events around
+// the launch: residual of 17^3 rows, B = 4, FP64 30 -> 15 us; of the seven levels
+// below 513^2 rows, B = 3, FP32 about 14 -> 11.8 us each. On the 513^2 level
+// itself the x loads, B times as many, cost more than they gain (the solve 13.9 ->
+// 14.3 ms).
+// The lines of block_split: products with a thread per row and with this, us in
+// FP64 and in FP32.
+//   9 blocks a row,  B = 2: 40,401 rows 10.1 10.3, 9.5 8.8; 57,600 10.5 11.3, 8.7 9.3
+//                    B = 3: 75,625 14.3 14.0, 12.1 11.9; 96,100 14.5 15.7, 12.2 12.2
+//                    B = 4: 25,600 16.0 15.5, 14.6 12.2; 40,401 16.3 18.2, 13.0 12.5
+//   27 blocks a row, B = 2: 68,921 14.7 14.8, 12.9 12.0; 97,336 16.5 22.3, 12.9 14.0
+//                    B = 3: 97,336 57.7 37.8, 41.4 20.9
+//                    B = 4: 97,336 78.4 68.6, 65.5 41.9; 117,649 was not split
+inline bool
+block_split(int64_t rows, int blocks_per_row, int B)
+{
+  if (blocks_per_row > 16)
+    return rows <= (B == 2 ? 70000 : 100000);
+  return rows <= (B == 2 ? 48000 : B == 3 ? 80000 : 32768);
+}
 template<int MODE, int B, class TV, class TX, class TO, bool PAT>
 __global__ void __launch_bounds__(kSpmvThreads, 2)
 k_bspmv_split(SellView<TV> A, const TX* __restrict__ x, TO* __restrict__ y,

@@ -771,7 +771,7 @@ bspmv(Context& c, const Level& L, const Sell& S, const TX* x, TO* y, const TO* b
 {
   const SellView<TV> A = view<TV>(S, sell_vals<TV>(S));
   if constexpr (MODE != kJacobi) { // that mode needs a row's components together
-    if (S.n <= kBlockSplitRows) {
+    if (block_split(S.n, S.wmax, B)) {
       const int nb = blocks_for(int64_t(S.nslices) * B * kSlice, kSpmvThreads);
       launch(c, S.pat ? k_bspmv_split<MODE, B, TV, TX, TO, true>
                       : k_bspmv_split<MODE, B, TV, TX, TO, false>,

@@ -158,7 +158,7 @@ const double* Emit<T>::resid_mean(int l, const T* u, T* out, const T* b)
   if (L.B > 1) {
     check_pf_scratch(L);
     const SellView<T> A = view<T>(S, sell_vals<T>(S));
-    const bool split = S.n <= kBlockSplitRows;
+    const bool split = block_split(S.n, S.wmax, L.B);
     const int nb = split ? blocks_for(int64_t(S.nslices) * S.B * kSlice, kSpmvThreads)
                          : blocks_for(S.n, kSpmvThreads);
 #define GB_RM(BB, PP)                                                                 \
