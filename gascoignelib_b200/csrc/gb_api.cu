@@ -942,17 +942,8 @@ gb_restrict_zero(gb_ctx* ctx, int lvl, int coarse_id, int fine_id)
         launch(*ctx, k_restrict<double>, nb, 256, T.nc, tp, te, f, cc, nm,
                (const double*)nullptr, (double*)nullptr, 0.0);
       break;
-    case 2:
-      launch(*ctx, k_restrict_b<double, 2>, blocks_for(int64_t(T.nc) * 2, 256), 256, T.nc, tp, te, f, cc, nm, -1,
-             (const double*)nullptr);
-      break;
-    case 3:
-      launch(*ctx, k_restrict_b<double, 3>, blocks_for(int64_t(T.nc) * 3, 256), 256, T.nc, tp, te, f, cc, nm, -1,
-             (const double*)nullptr);
-      break;
     default:
-      launch(*ctx, k_restrict_b<double, 4>, blocks_for(int64_t(T.nc) * 4, 256), 256, T.nc, tp, te, f, cc, nm, -1,
-             (const double*)nullptr);
+      block_restrict<double>(*ctx, B, T, f, cc, nm, -1, nullptr);
   }
   GB_API_END
 }
@@ -974,14 +965,8 @@ gb_prolongate_add(gb_ctx* ctx, int lvl, int fine_id, int coarse_id)
     case 1:
       launch(*ctx, k_prolong<0, double>, nb, 256, T.nf, tp, te, cc, f, nm, 1.0);
       break;
-    case 2:
-      launch(*ctx, k_prolong_b<0, double, 2>, blocks_for(int64_t(T.nf) * 2, 256), 256, T.nf, tp, te, cc, f, nm, 1.0);
-      break;
-    case 3:
-      launch(*ctx, k_prolong_b<0, double, 3>, blocks_for(int64_t(T.nf) * 3, 256), 256, T.nf, tp, te, cc, f, nm, 1.0);
-      break;
     default:
-      launch(*ctx, k_prolong_b<0, double, 4>, blocks_for(int64_t(T.nf) * 4, 256), 256, T.nf, tp, te, cc, f, nm, 1.0);
+      block_prolong<0, double>(*ctx, B, T, cc, f, nm, 1.0);
   }
   GB_API_END
 }

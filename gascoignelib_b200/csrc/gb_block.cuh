@@ -341,82 +341,121 @@ k_block_jacobi_apply(int n, const TV* __restrict__ dinv, const T* __restrict__ h
   }
 }
 
-// Block transfers: the scalar tables applied to each of the B components, one
-// thread per node and component (the B threads of a node read B consecutive
-// values), eight entries in flight. The sum runs over the entries in order from
-// acc (0, or the target for an in-place add: the weights are powers of two, so
-// each fused add rounds like the reference's y += w x). Component pc is read
-// minus smean.
-template<class T, int B>
-__device__ __forceinline__ T
-transfer_dof(const int* __restrict__ tsp, const uint32_t* __restrict__ tent,
-             const T* __restrict__ src, int i, int c, T acc, bool sub = false,
-             double smean = 0.0)
+// Block transfers: the scalar tables applied to each of the B components. A thread
+// takes C components of a node: one (the B threads of a node read B consecutive
+// values, eight entries in flight), or all B. The sum runs over the entries in order
+// from acc (0, or the target for an in-place add: the weights are powers of two, so
+// each fused add rounds like the reference's y += w x), so both give the same bits.
+// Component pc is read minus smean.
+// One component per thread hides the entries' latency on small levels, and reads
+// every entry B times: up to kDofThreadRows nodes. Thread per node and per component,
+// us with events around the launch, B = 3 in 2D, FP64:
+//   prolongation to   66,049 nodes 10.3 8.6; 263,169 10.6 17.8; 1,050,625 20.8 46.3
+//   restriction to    66,049 nodes 14.7 12.6; 263,169 16.7 26.4
+//   the Vanka averages of a cycle on two levels (4 on the finer, 1 on the coarser),
+//                     66,049 nodes 62 61; 263,169 88 104; 1,050,625 194 294
+// B = 4 in 3D: prolongation to 117,649 nodes 12.7 14.1, averages 82 86.
+constexpr int64_t kDofThreadRows = 70000;
+
+template<class T, int B, int C>
+__device__ __forceinline__ void
+transfer_row_b(const int* __restrict__ tsp, const uint32_t* __restrict__ tent,
+               const T* __restrict__ src, int i, int c0, T (&acc)[C], int pc = -1,
+               double smean = 0.0)
 {
   const int beg = __ldg(tsp + (i >> 5));
   const int w = (__ldg(tsp + (i >> 5) + 1) - beg) >> 5;
   const uint32_t* ep = tent + beg + (i & 31);
-  for (int j0 = 0; j0 < w; j0 += 8) {
-    const uint32_t* pe[8];
+  if constexpr (C > 1) {
+    for (int j = 0; j < w; ++j) {
+      const uint32_t e = __ldg(ep + j * kSlice);
+      const T wgt = wcode<T>(e);
+      const T* sp = src + int64_t(e & kIdxMask) * B;
 #pragma unroll
-    for (int q = 0; q < 8; ++q)
-      pe[q] = ep + min(j0 + q, w - 1) * kSlice;
-    uint32_t e[8];
-    ld8(e, pe);
-    const T* ps[8];
-#pragma unroll
-    for (int q = 0; q < 8; ++q)
-      ps[q] = src + int64_t(e[q] & kIdxMask) * B + c;
-    T f[8];
-    ld8(f, ps);
-#pragma unroll
-    for (int q = 0; q < 8; ++q)
-      if (j0 + q < w) {
-        const T sv = sub ? static_cast<T>(static_cast<double>(f[q]) - smean) : f[q];
-        acc = fma(wcode<T>(e[q]), sv, acc);
+      for (int c = 0; c < C; ++c) {
+        const T sv = c == pc ? static_cast<T>(static_cast<double>(__ldg(sp + c)) - smean)
+                             : __ldg(sp + c);
+        acc[c] = fma(wgt, sv, acc[c]);
       }
+    }
+  } else {
+    for (int j0 = 0; j0 < w; j0 += 8) {
+      const uint32_t* pe[8];
+#pragma unroll
+      for (int q = 0; q < 8; ++q)
+        pe[q] = ep + min(j0 + q, w - 1) * kSlice;
+      uint32_t e[8];
+      ld8(e, pe);
+      const T* ps[8];
+#pragma unroll
+      for (int q = 0; q < 8; ++q)
+        ps[q] = src + int64_t(e[q] & kIdxMask) * B + c0;
+      T f[8];
+      ld8(f, ps);
+#pragma unroll
+      for (int q = 0; q < 8; ++q)
+        if (j0 + q < w) {
+          const T sv = c0 == pc ? static_cast<T>(static_cast<double>(f[q]) - smean) : f[q];
+          acc[0] = fma(wcode<T>(e[q]), sv, acc[0]);
+        }
+    }
   }
-  return acc;
 }
 
 // fine's component pc is read minus *smean when smean is set (the filtered
 // residual of MatrixResidual, restricted).
-template<class T, int B>
+template<class T, int B, int C>
 __global__ void __launch_bounds__(256)
 k_restrict_b(int nc, const int* __restrict__ tsp, const uint32_t* __restrict__ tent,
              const T* __restrict__ fine, T* __restrict__ coarse,
-             const uint8_t* __restrict__ cdir, int pc = -1,
-             const double* __restrict__ smean = nullptr)
+             const uint8_t* __restrict__ cdir, int pc, const double* __restrict__ smean)
 {
   GB_PDL_ENTRY();
-  const int64_t d = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
-  const int i = static_cast<int>(d / B), c = static_cast<int>(d % B);
+  constexpr int S = B / C; // threads of a node
+  const int64_t t = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
+  const int i = static_cast<int>(t / S), c0 = static_cast<int>(t % S);
   if (i >= nc)
     return;
-  const T acc = transfer_dof<T, B>(tsp, tent, fine, i, c, T(0), smean && c == pc,
-                                   smean ? *smean : 0.0);
-  coarse[d] = (cdir && cdir[d]) ? T(0) : acc;
+  T acc[C];
+#pragma unroll
+  for (int c = 0; c < C; ++c)
+    acc[c] = T(0);
+  transfer_row_b<T, B, C>(tsp, tent, fine, i, c0, acc, smean ? pc : -1, smean ? *smean : 0.0);
+#pragma unroll
+  for (int c = 0; c < C; ++c) {
+    const int64_t d = int64_t(i) * B + c0 + c;
+    coarse[d] = (cdir && cdir[d]) ? T(0) : acc[c];
+  }
 }
 
-template<int MODE, class T, int B>
+template<int MODE, class T, int B, int C>
 __global__ void __launch_bounds__(256)
 k_prolong_b(int nf, const int* __restrict__ tsp, const uint32_t* __restrict__ tent,
             const T* __restrict__ coarse, T* __restrict__ fine,
             const uint8_t* __restrict__ fdir, double mgomega)
 {
   GB_PDL_ENTRY();
-  const int64_t d = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
-  const int i = static_cast<int>(d / B), c = static_cast<int>(d % B);
+  constexpr int S = B / C;
+  const int64_t t = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
+  const int i = static_cast<int>(t / S), c0 = static_cast<int>(t % S);
   if (i >= nf)
     return;
-  if (MODE == 0) {
-    fine[d] = transfer_dof<T, B>(tsp, tent, coarse, i, c, fine[d]);
-    return;
+  const int64_t d0 = int64_t(i) * B + c0;
+  T acc[C];
+#pragma unroll
+  for (int c = 0; c < C; ++c)
+    acc[c] = MODE == 0 ? fine[d0 + c] : T(0);
+  transfer_row_b<T, B, C>(tsp, tent, coarse, i, c0, acc);
+#pragma unroll
+  for (int c = 0; c < C; ++c) {
+    const int64_t d = d0 + c;
+    if (MODE == 0) {
+      fine[d] = acc[c];
+    } else {
+      const T a = (fdir && fdir[d]) ? T(0) : acc[c];
+      fine[d] = fine[d] + static_cast<T>(mgomega) * a;
+    }
   }
-  T a = transfer_dof<T, B>(tsp, tent, coarse, i, c, T(0));
-  if (fdir && fdir[d])
-    a = T(0);
-  fine[d] = fine[d] + static_cast<T>(mgomega) * a;
 }
 
 // ------------------------------------------------------ pressure filter
@@ -724,10 +763,11 @@ k_vanka_inv_ct(int npatch, int B, const int* __restrict__ pn, const TL* __restri
 }
 
 // u(i, c) = (u_zero ? 0 : u(i, c)) + omega * ((sum over the node's patches of
-// their solution at (i, c)) * (1 / count)), a thread per node and component.
-// ent packs (patch, local node): patch * 32 + r (npp <= 27). Solution (patch p,
-// local dof q) at hout[p * M + q].
-template<int B, class T>
+// their solution at (i, c)) * (1 / count)), C components of a node per thread
+// (kDofThreadRows, the block transfers' rule; the same bits). ent packs (patch,
+// local node): patch * 32 + r (npp <= 27). Solution (patch p, local dof q) at
+// hout[p * M + q].
+template<int B, int C, class T>
 __global__ void __launch_bounds__(256)
 k_vanka_gather(int n, const int* __restrict__ nptr, const int* __restrict__ ent,
                const T* __restrict__ hout, int M, T* __restrict__ u, double omega,
@@ -735,35 +775,49 @@ k_vanka_gather(int n, const int* __restrict__ nptr, const int* __restrict__ ent,
 {
   GB_PDL_ENTRY();
   using TA = typename Acc<T, T>::type;
+  constexpr int S = B / C;         // threads of a node
+  constexpr int F = C == 1 ? 4 : 1; // patches' values in flight
   __shared__ double sh[32];
-  const int64_t d = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
-  const int i = static_cast<int>(d / B), c = static_cast<int>(d % B);
+  const int64_t t = blockIdx.x * int64_t(blockDim.x) + threadIdx.x;
+  const int i = static_cast<int>(t / S), c0 = static_cast<int>(t % S);
   double wv = 0.0;
   if (i < n) {
     const int k0 = __ldg(nptr + i), k1 = __ldg(nptr + i + 1);
-    TA acc = TA(0);
-    for (int k = k0; k < k1; k += 4) { // four patches' values in flight
-      int e[4];
+    TA acc[C];
 #pragma unroll
-      for (int q = 0; q < 4; ++q)
+    for (int c = 0; c < C; ++c)
+      acc[c] = TA(0);
+    for (int k = k0; k < k1; k += F) {
+      int e[F];
+#pragma unroll
+      for (int q = 0; q < F; ++q)
         e[q] = k + q < k1 ? __ldg(ent + k + q) : -1;
-      TA v[4];
+      TA v[F][C];
 #pragma unroll
-      for (int q = 0; q < 4; ++q)
-        v[q] = e[q] >= 0
-                 ? static_cast<TA>(hout[int64_t(e[q] >> 5) * M + (e[q] & 31) * B + c])
-                 : TA(0);
+      for (int q = 0; q < F; ++q)
 #pragma unroll
-      for (int q = 0; q < 4; ++q)
+        for (int c = 0; c < C; ++c)
+          v[q][c] =
+            e[q] >= 0
+              ? static_cast<TA>(hout[int64_t(e[q] >> 5) * M + (e[q] & 31) * B + c0 + c])
+              : TA(0);
+#pragma unroll
+      for (int q = 0; q < F; ++q)
         if (e[q] >= 0)
-          acc += v[q];
+#pragma unroll
+          for (int c = 0; c < C; ++c)
+            acc[c] += v[q][c];
     }
     const TA sc = TA(1) / static_cast<TA>(k1 - k0);
-    const TA base = u_zero ? TA(0) : static_cast<TA>(u[d]);
-    const T un = static_cast<T>(base + static_cast<TA>(omega) * (acc * sc));
-    u[d] = un;
-    if (pf.w && c == pf.pc)
-      wv = static_cast<double>(un) * pf.w[i];
+#pragma unroll
+    for (int c = 0; c < C; ++c) {
+      const int64_t d = int64_t(i) * B + c0 + c;
+      const TA base = u_zero ? TA(0) : static_cast<TA>(u[d]);
+      const T un = static_cast<T>(base + static_cast<TA>(omega) * (acc[c] * sc));
+      u[d] = un;
+      if (pf.w && c0 + c == pf.pc)
+        wv = static_cast<double>(un) * pf.w[i];
+    }
   }
   if (pf.w) {
     wv = block_sum(wv, sh);

@@ -764,6 +764,45 @@ ilu_in_cluster(const Level& L)
 }
 void ensure_work(Context& c);
 
+// Transfers of block levels (B >= 2).
+template<class T>
+inline void
+block_restrict(Context& c, int B, const Transfer& Tr, const T* fine, T* coarse,
+               const uint8_t* cdir, int pc, const double* smean)
+{
+  auto run = [&](auto block) {
+    constexpr int BB = decltype(block)::value;
+    const bool dofs = Tr.nc <= kDofThreadRows;
+    launch(c, dofs ? k_restrict_b<T, BB, 1> : k_restrict_b<T, BB, BB>,
+           blocks_for(int64_t(Tr.nc) * (dofs ? BB : 1), 256), 256, Tr.nc, Tr.rptr.p, Tr.rent.p,
+           fine, coarse, cdir, pc, smean);
+  };
+  switch (B) {
+    case 2: run(std::integral_constant<int, 2>{}); break;
+    case 3: run(std::integral_constant<int, 3>{}); break;
+    default: run(std::integral_constant<int, 4>{});
+  }
+}
+
+template<int MODE, class T>
+inline void
+block_prolong(Context& c, int B, const Transfer& Tr, const T* coarse, T* fine,
+              const uint8_t* fdir, double mgomega)
+{
+  auto run = [&](auto block) {
+    constexpr int BB = decltype(block)::value;
+    const bool dofs = Tr.nf <= kDofThreadRows;
+    launch(c, dofs ? k_prolong_b<MODE, T, BB, 1> : k_prolong_b<MODE, T, BB, BB>,
+           blocks_for(int64_t(Tr.nf) * (dofs ? BB : 1), 256), 256, Tr.nf, Tr.pptr.p, Tr.pent.p,
+           coarse, fine, fdir, mgomega);
+  };
+  switch (B) {
+    case 2: run(std::integral_constant<int, 2>{}); break;
+    case 3: run(std::integral_constant<int, 3>{}); break;
+    default: run(std::integral_constant<int, 4>{});
+  }
+}
+
 template<int MODE, int B, class TV, class TX, class TO>
 inline void
 bspmv(Context& c, const Level& L, const Sell& S, const TX* x, TO* y, const TO* b,

@@ -91,27 +91,18 @@ void Emit<T>::vanka(int l, const T* h, T* u, bool u_zero, const double* hmean)
     }
   }
   const PfArgs pf = weighted_mean_args(L);
-  const int nb = blocks_for(L.ndof(), 256);
+  auto gather = [&](auto block) {
+    constexpr int B = decltype(block)::value;
+    const bool dofs = L.n <= kDofThreadRows;
+    launch(c, dofs ? k_vanka_gather<B, 1, T> : k_vanka_gather<B, B, T>,
+           blocks_for(dofs ? L.ndof() : L.n, 256), 256, (int)L.n, (const int*)L.vk_nptr.p,
+           (const int*)L.vk_ent.p, (const T*)out, L.vk_M, u, c.params.omega, int(u_zero), pf);
+  };
   switch (L.B) {
-    case 1:
-      launch(c, k_vanka_gather<1, T>, nb, 256, (int)L.n, (const int*)L.vk_nptr.p,
-             (const int*)L.vk_ent.p, (const T*)out, L.vk_M, u, c.params.omega,
-             int(u_zero), pf);
-      break;
-    case 2:
-      launch(c, k_vanka_gather<2, T>, nb, 256, (int)L.n, (const int*)L.vk_nptr.p,
-             (const int*)L.vk_ent.p, (const T*)out, L.vk_M, u, c.params.omega,
-             int(u_zero), pf);
-      break;
-    case 3:
-      launch(c, k_vanka_gather<3, T>, nb, 256, (int)L.n, (const int*)L.vk_nptr.p,
-             (const int*)L.vk_ent.p, (const T*)out, L.vk_M, u, c.params.omega,
-             int(u_zero), pf);
-      break;
-    default:
-      launch(c, k_vanka_gather<4, T>, nb, 256, (int)L.n, (const int*)L.vk_nptr.p,
-             (const int*)L.vk_ent.p, (const T*)out, L.vk_M, u, c.params.omega,
-             int(u_zero), pf);
+    case 1: gather(std::integral_constant<int, 1>{}); break;
+    case 2: gather(std::integral_constant<int, 2>{}); break;
+    case 3: gather(std::integral_constant<int, 3>{}); break;
+    default: gather(std::integral_constant<int, 4>{});
   }
 }
 
@@ -438,18 +429,9 @@ void Emit<T>::restrict_to(int l, const T* fine, T* coarse, const double* smean, 
         launch(c, k_restrict<T>, nb, 256, Tr.nc, Tr.rptr.p, Tr.rent.p, fine, coarse, cm, dv,
                u1, c.params.omega);
       break;
-    case 2:
-      GB_REQUIRE(!u1, GB_EINVAL, "fused first sweep on a block level");
-      launch(c, k_restrict_b<T, 2>, blocks_for(int64_t(Tr.nc) * 2, 256), 256, Tr.nc, Tr.rptr.p, Tr.rent.p, fine, coarse, cm,
-             pf_comp(c.L[l + 1]), smean);
-      break;
-    case 3:
-      launch(c, k_restrict_b<T, 3>, blocks_for(int64_t(Tr.nc) * 3, 256), 256, Tr.nc, Tr.rptr.p, Tr.rent.p, fine, coarse, cm,
-             pf_comp(c.L[l + 1]), smean);
-      break;
     default:
-      launch(c, k_restrict_b<T, 4>, blocks_for(int64_t(Tr.nc) * 4, 256), 256, Tr.nc, Tr.rptr.p, Tr.rent.p, fine, coarse, cm,
-             pf_comp(c.L[l + 1]), smean);
+      GB_REQUIRE(!u1, GB_EINVAL, "fused first sweep on a block level");
+      block_restrict<T>(c, c.L[l].B, Tr, fine, coarse, cm, pf_comp(c.L[l + 1]), smean);
   }
 }
 
@@ -510,17 +492,8 @@ void Emit<T>::prolong(int l, const T* coarse, T* fine)
     case 1:
       launch(c, k_prolong<1, T>, nb, 256, Tr.nf, Tr.pptr.p, Tr.pent.p, coarse, fine, fm, mw);
       break;
-    case 2:
-      launch(c, k_prolong_b<1, T, 2>, blocks_for(int64_t(Tr.nf) * 2, 256), 256, Tr.nf, Tr.pptr.p, Tr.pent.p, coarse, fine,
-             fm, mw);
-      break;
-    case 3:
-      launch(c, k_prolong_b<1, T, 3>, blocks_for(int64_t(Tr.nf) * 3, 256), 256, Tr.nf, Tr.pptr.p, Tr.pent.p, coarse, fine,
-             fm, mw);
-      break;
     default:
-      launch(c, k_prolong_b<1, T, 4>, blocks_for(int64_t(Tr.nf) * 4, 256), 256, Tr.nf, Tr.pptr.p, Tr.pent.p, coarse, fine,
-             fm, mw);
+      block_prolong<1, T>(c, c.L[l + 1].B, Tr, coarse, fine, fm, mw);
   }
 }
 
