@@ -34,7 +34,7 @@ gb_ctx_create(gb_ctx** out, int device)
     if (const char* e = getenv("GB_ILU_CTA_ROWS"))
       ctx->ilu_cta_rows = std::max(0, atoi(e)), ctx->ilu_cluster = false;
     if (const char* e = getenv("GB_EXACT_CTAS"))
-      ctx->exact_ctas = std::min(std::max(0, atoi(e)), kExactMaxCtas);
+      ctx->exact_ctas = std::min(std::max(0, atoi(e)), kExactMaxCtas), ctx->exact_any = true;
     if (const char* e = getenv("GB_VANKA_HOST"))
       ctx->vanka_host = atoi(e) != 0;
     if (const char* e = getenv("GB_CLUSTER"))

@@ -473,8 +473,10 @@ struct gb_ctx
   // GB_ILU_CTA_ROWS asks for the level launches)
   bool ilu_cluster = true;
   // CTAs of the cluster of the coarsest level's sweeps (GB_EXACT_CTAS; 0: a
-  // launch per sweep; -1: the largest the device runs)
+  // launch per sweep; -1: the largest the device runs), and whether it takes every
+  // level that fits (GB_EXACT_CTAS set) or those of exact_rows
   int exact_ctas = -1;
+  bool exact_any = false;
   int ilu_max_ctas = 0; // largest cluster of k_ilu_cluster (0: not queried)
   // GB_CLUSTER=1: the levels of at most cluster_rows dofs below the finest
   // (and above the single-CTA coarse levels) as one op program run by one

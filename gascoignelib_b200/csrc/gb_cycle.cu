@@ -368,7 +368,8 @@ bool Emit<T>::exact_sweeps(int l, int niter, T* u, const T* b, bool u_zero)
   const Sell& A = opA(c, L);
   // Levels up to kCoarseMaxRows have their dense map or op program; two sweeps
   // are not worth the copy of the matrix.
-  if (rec || L.B != 1 || L.n <= kCoarseMaxRows || L.n > 65535 || niter < 3)
+  if (rec || L.B != 1 || L.n <= kCoarseMaxRows || L.n > 65535 || niter < 3 ||
+      (!c.exact_any && L.n > exact_rows<T>(A.wmax)))
     return false;
   const int ctas = c.exact_ctas;
   if (ctas <= 0)

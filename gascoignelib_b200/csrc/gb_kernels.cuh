@@ -2027,7 +2027,7 @@ cluster_barrier()
 // ahead that another CTA's threads have read their partial sums, and a wait that
 // ran out would leave values under way.) Solves with a launch per sweep and with
 // this: 80^3 Q2 cells 41.8 and 41.6 ms, 40^3 Q2 cells with a refined ball 43.5
-// and 43.1 ms, 56^3 Q1 cells (left) 1.76 and 1.74 ms.
+// and 43.1 ms. Where it is taken: exact_rows.
 // Why nothing is overwritten while it is read: a sweep's last reads of `part`
 // and of the old copy of x come before its cluster barrier, for every thread of
 // every CTA, and the next sweep, which is the next to write `part` and the old
@@ -2044,6 +2044,28 @@ cluster_barrier()
 constexpr int kExactWarps = 32;
 constexpr int kExactMaxCtas = 16;
 constexpr size_t kExactBytes = 220 * 1024; // shared memory per CTA
+
+// The most rows of a coarsest level whose sweeps run in the cluster, by its longest
+// row. A sweep there grows with the entries per CTA (and, where the rows' order by
+// length makes a slice's rows far apart, with bank conflicts of their x), a launch
+// stays at 2 to 3 us within a solver graph. What the cluster adds to a step of the
+// flexible solve, nine sweeps, us in FP64 and in FP32:
+//   9 entries (Q1, 2D): 1,225 rows -3.0 -2.7; 1,681 -2.7 -2.2; 2,401 -0.2 0.0;
+//                       4,225 +4.3 +1.7; 8,281 +23 +12
+//   25 (Q2, 2D):        1,225 +1.7 -4.3; 2,401 +19 +4.8; 4,225 +49 +22
+//   27 (Q1, 3D):        1,331 -6.5 -7.5; 2,197 -2.3 -4.2; 3,375 -0.7 (another
+//                       right-hand side: +1.2) -3.5; 4,913 +8.8 +3.5
+//   125 (Q2, 3D):       1,331 -5.2 -4.6; 2,197 +12 +5.2
+template<class T>
+constexpr int
+exact_rows(int longest_row)
+{
+  const bool fp64 = sizeof(T) == 8;
+  return longest_row <= 16   ? 2048
+         : longest_row <= 26 ? (fp64 ? 0 : 1500)
+         : longest_row <= 32 ? (fp64 ? 2700 : 3700)
+                             : 1500;
+}
 
 // x twice, the partial sums, the entries' values and columns
 template<class T>
