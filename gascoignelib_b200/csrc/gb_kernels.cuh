@@ -280,22 +280,34 @@ k_spmv(SellView<TV> A, const TX* __restrict__ x, TO* __restrict__ y,
   }
 }
 
-// k_spmv for long rows: kPartWarps warps (a CTA) share a slice and take its
-// columns in turn, four at a time (the 16-byte offset loads); a row's partial
-// sums are added in the warps' order. Which warp takes an entry depends on its
-// place in the row alone, so the slots' order leaves the result unchanged, but
-// the sum is not the sequential one of k_spmv: levels with rows of at most
-// kPartMinWidth entries, which the op programs of the multi-CTA cycle also run,
-// never take this form.
+// k_spmv for long rows: kPartWarps warps (a CTA) share a slice's loads, one of them
+// does its sums. The warps copy the values and the gathered x of a stage of columns
+// to shared memory (asynchronous copies: no registers wait for them, so both stages
+// are in flight at once); then warp 0 sums each row in its entries' order, as
+// k_spmv does: the same bits. What bounds it is one round of load latencies and the
+// chain of a row's multiply-adds.
 constexpr int kPartWarps = 4;
+template<class T>
+constexpr int kPartCols = sizeof(T) == 8 ? 32 : 64; // columns of a stage: 16 KB
 // Taken up to kPartMaxRows rows, where one thread per row leaves the GPU idle:
-// 9,261 Q2 rows with events around the launch: FP32 sweep 11.0 -> 8.9 us, FP64
-// product 15.6 -> 9.4 us. At 68,921 rows it is no faster (FP64 sweep 14.8 ->
-// 16.7 us), at 102,773 slower (28.0 -> 34.4 us).
+// Q2 rows in 3D with events around the launch, k_spmv and this, FP64 sweep, FP64
+// product, FP32 sweep: 4,913 rows 14.0 10.7, 16.3 10.1, 13.2 10.7 us; 9,261 14.2
+// 11.1, 15.1 9.2, 12.1 9.5; 19,683 14.1 13.2, 16.3 13.1, 13.6 12.2; 29,791 14.3 14.7,
+// 16.4 14.2, 13.4 14.2.
 constexpr int kPartMinWidth = 32;
-constexpr int kPartMaxRows = 32768;
+constexpr int kPartMaxRows = 20000;
+
+// N bytes (4 or 8) from global to shared memory, with the thread's next commit.
+template<int N>
+__device__ __forceinline__ void
+copy_async(uint32_t to, const void* from)
+{
+  asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(to), "l"(from), "n"(N)
+               : "memory");
+}
+
 template<int MODE, class TV, class TX, class TO, int CM>
-__global__ void __launch_bounds__(kPartWarps * 32, sizeof(TV) == 4 ? 10 : 8)
+__global__ void __launch_bounds__(kPartWarps * 32, 7)
 k_spmv_parts(SellView<TV> A, const TX* __restrict__ x, TO* __restrict__ y,
              const TO* __restrict__ b, const TV* __restrict__ dinv,
              const uint8_t* __restrict__ dirmask, double alpha_,
@@ -304,54 +316,65 @@ k_spmv_parts(SellView<TV> A, const TX* __restrict__ x, TO* __restrict__ y,
   GB_PDL_ENTRY();
   using TA = typename Acc<TV, TO>::type;
   constexpr bool NEG = MODE == kResid || MODE == kResidDir || MODE == kJacobi;
-  constexpr int C = 16; // entries in flight
-  __shared__ TA part[kPartWarps][kSlice];
+  constexpr int C = kPartCols<TV>;
+  __shared__ TV sv[2][C][kSlice];
+  __shared__ TX sx[2][C][kSlice];
   const int s = blockIdx.x, lane = threadIdx.x & 31, q = threadIdx.x >> 5;
   const int slot = s * kSlice + lane;
   const bool ok = slot < A.n;
   const int row = !ok ? 0 : A.perm ? __ldg(A.perm + slot) : slot;
   const int beg = A.sptr[s];
   const int w = (A.sptr[s + 1] - beg) >> 5;
-  TA acc = TA(0);
-  if (ok) {
-    const TV* vp = A.val + beg + lane;
-    const int* cp = CM == kColPat ? (A.ptab + int(A.pid[row]) * A.W) : (A.col + beg + lane);
-    const int16_t* hp = A.c16 + beg + lane;
-    for (int j0 = 4 * q; j0 < w; j0 += C * kPartWarps) {
-      TA av[C], xv[C];
-      int4 o4;
+  const TV* vp = A.val + beg + lane;
+  const int* cp = CM == kColPat ? (A.ptab + int(A.pid[row]) * A.W) : (A.col + beg + lane);
+  const int16_t* hp = A.c16 + beg + lane;
+  const uint32_t tv = static_cast<uint32_t>(__cvta_generic_to_shared(&sv[0][0][lane]));
+  const uint32_t tx = static_cast<uint32_t>(__cvta_generic_to_shared(&sx[0][0][lane]));
+  // this warp's columns of the stage that begins at j0, four at a time
+  auto issue = [&](int p, int j0) {
 #pragma unroll
-      for (int k = 0; k < C; ++k) {
-        const int j = j0 + k / 4 * (4 * kPartWarps) + k % 4;
-        if (j < w) {
-          if (CM == kColPat && k % 4 == 0)
-            o4 = ldg(reinterpret_cast<const int4*>(cp + j));
-          const int c = CM == kColPat
-                          ? row + (k % 4 == 0 ? o4.x : k % 4 == 1 ? o4.y : k % 4 == 2 ? o4.z : o4.w)
-                          : CM == kColOff16 ? row + int(ldg(hp + j * kSlice))
-                                            : ldg(cp + j * kSlice);
-          av[k] = static_cast<TA>(ldg(vp + j * kSlice));
-          xv[k] = static_cast<TA>(ldg(x + c));
-        } else {
-          av[k] = TA(0);
-          xv[k] = TA(0);
+    for (int k0 = 0; k0 < C; k0 += 4 * kPartWarps) {
+      const int k = k0 + 4 * q;
+      int4 o4;
+      if (CM == kColPat && ok && j0 + k < w)
+        o4 = ldg(reinterpret_cast<const int4*>(cp + j0 + k));
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const int j = j0 + k + u;
+        if (ok && j < w) {
+          const int c = CM == kColPat ? row + (u == 0 ? o4.x : u == 1 ? o4.y : u == 2 ? o4.z : o4.w)
+                        : CM == kColOff16 ? row + int(ldg(hp + j * kSlice))
+                                          : ldg(cp + j * kSlice);
+          const uint32_t at = uint32_t((p * C + k + u) * kSlice);
+          copy_async<sizeof(TV)>(tv + at * uint32_t(sizeof(TV)), vp + j * kSlice);
+          copy_async<sizeof(TX)>(tx + at * uint32_t(sizeof(TX)), x + c);
         }
       }
-#pragma unroll
-      for (int k = 0; k < C; ++k)
-        acc = fma(av[k], xv[k], acc);
     }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  issue(0, 0);
+  issue(1, C);
+  TA acc = NEG && ok && q == 0 ? static_cast<TA>(b[row]) : TA(0);
+  for (int j0 = 0, p = 0; j0 < w; j0 += C, p ^= 1) {
+    // this thread's part of the stage has come, then every thread's
+    asm volatile("cp.async.wait_group 1;" ::: "memory");
+    __syncthreads();
+    if (q == 0 && ok) {
+      const int cnt = min(C, w - j0);
+#pragma unroll 8
+      for (int k = 0; k < cnt; ++k) {
+        const TA av = static_cast<TA>(sv[p][k][lane]), xv = static_cast<TA>(sx[p][k][lane]);
+        acc = NEG ? fma(-av, xv, acc) : fma(av, xv, acc);
+      }
+    }
+    if (j0 + 2 * C < w)
+      __syncthreads(); // the stage has been read
+    issue(p, j0 + 2 * C);
   }
-  part[q][lane] = acc;
-  __syncthreads();
   if (q != 0 || !ok)
     return;
-#pragma unroll
-  for (int k = 1; k < kPartWarps; ++k)
-    acc += part[k][lane];
   const TA alpha = static_cast<TA>(alpha_);
-  if (NEG)
-    acc = static_cast<TA>(b[row]) - acc;
   if (yidx) {
     const int64_t jj = *yidx;
     xcopy[jj * ystride + row] = x[row];
