@@ -283,12 +283,15 @@ k_spmv(SellView<TV> A, const TX* __restrict__ x, TO* __restrict__ y,
 // k_spmv for long rows: kPartWarps warps (a CTA) share a slice's loads, one of them
 // does its sums. The warps copy the values and the gathered x of a stage of columns
 // to shared memory (asynchronous copies: no registers wait for them, so both stages
-// are in flight at once); then warp 0 sums each row in its entries' order, as
-// k_spmv does: the same bits. What bounds it is one round of load latencies and the
-// chain of a row's multiply-adds.
+// are in flight at once; their column indices are all loaded before the first copy);
+// then warp 0 sums each row in its entries' order, with the zeros behind its end, as
+// k_spmv does: the same bits. What bounds it is one round of load latencies (index,
+// then x) and the chain of a row's multiply-adds, unrolled over the whole stage (FP32,
+// steps of a solve with 1,331 coarsest Q2 rows: stages of 32 columns 84.4 us, of 64
+// 80.5 us; rolled by 8: 86 us).
 constexpr int kPartWarps = 4;
 template<class T>
-constexpr int kPartCols = sizeof(T) == 8 ? 32 : 64; // columns of a stage: 16 KB
+constexpr int kPartCols = sizeof(T) == 8 ? 32 : 64; // columns of a stage
 // Taken up to kPartMaxRows rows, where one thread per row leaves the GPU idle:
 // Q2 rows in 3D with events around the launch, k_spmv and this, FP64 sweep, FP64
 // product, FP32 sweep: 4,913 rows 14.0 10.7, 16.3 10.1, 13.2 10.7 us; 9,261 14.2
@@ -297,12 +300,14 @@ constexpr int kPartCols = sizeof(T) == 8 ? 32 : 64; // columns of a stage: 16 KB
 constexpr int kPartMinWidth = 32;
 constexpr int kPartMaxRows = 20000;
 
-// N bytes (4 or 8) from global to shared memory, with the thread's next commit.
-template<int N>
+// A value of 4 or 8 bytes from global to shared memory with the thread's next
+// commit, or (not `there`) a 0, with nothing read.
+template<class T>
 __device__ __forceinline__ void
-copy_async(uint32_t to, const void* from)
+copy_async(uint32_t to, const T* from, bool there)
 {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(to), "l"(from), "n"(N)
+  asm volatile("cp.async.ca.shared.global [%0], [%1], %2, %3;" ::"r"(to), "l"(from),
+               "n"(int(sizeof(T))), "r"(there ? int(sizeof(T)) : 0)
                : "memory");
 }
 
@@ -330,47 +335,66 @@ k_spmv_parts(SellView<TV> A, const TX* __restrict__ x, TO* __restrict__ y,
   const int16_t* hp = A.c16 + beg + lane;
   const uint32_t tv = static_cast<uint32_t>(__cvta_generic_to_shared(&sv[0][0][lane]));
   const uint32_t tx = static_cast<uint32_t>(__cvta_generic_to_shared(&sx[0][0][lane]));
-  // this warp's columns of the stage that begins at j0, four at a time
-  auto issue = [&](int p, int j0) {
+  // this warp's columns of the stage that begins at j0, four at a time: first all
+  // their indices, then the copies
+  constexpr int N = C / kPartWarps;
+  auto columns = [&](int j0, int (&c)[N]) {
 #pragma unroll
-    for (int k0 = 0; k0 < C; k0 += 4 * kPartWarps) {
-      const int k = k0 + 4 * q;
-      int4 o4;
-      if (CM == kColPat && ok && j0 + k < w)
-        o4 = ldg(reinterpret_cast<const int4*>(cp + j0 + k));
+    for (int i = 0; i < N; i += 4) {
+      const int j = j0 + i * kPartWarps + 4 * q;
+      if (CM == kColPat) {
+        int4 o = make_int4(0, 0, 0, 0);
+        if (ok && j < w)
+          o = ldg(reinterpret_cast<const int4*>(cp + j));
+        c[i] = row + o.x;
+        c[i + 1] = row + o.y;
+        c[i + 2] = row + o.z;
+        c[i + 3] = row + o.w;
+      } else {
 #pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        const int j = j0 + k + u;
-        if (ok && j < w) {
-          const int c = CM == kColPat ? row + (u == 0 ? o4.x : u == 1 ? o4.y : u == 2 ? o4.z : o4.w)
-                        : CM == kColOff16 ? row + int(ldg(hp + j * kSlice))
-                                          : ldg(cp + j * kSlice);
-          const uint32_t at = uint32_t((p * C + k + u) * kSlice);
-          copy_async<sizeof(TV)>(tv + at * uint32_t(sizeof(TV)), vp + j * kSlice);
-          copy_async<sizeof(TX)>(tx + at * uint32_t(sizeof(TX)), x + c);
-        }
+        for (int u = 0; u < 4; ++u)
+          c[i + u] = !ok || j + u >= w ? 0
+                     : CM == kColOff16 ? row + int(ldg(hp + (j + u) * kSlice))
+                                       : ldg(cp + (j + u) * kSlice);
       }
+    }
+  };
+  auto copy = [&](int p, int j0, const int (&c)[N]) {
+#pragma unroll
+    for (int i = 0; i < N; ++i) {
+      const int k = i / 4 * (4 * kPartWarps) + 4 * q + i % 4, j = j0 + k;
+      const bool there = ok && j < w;
+      const uint32_t at = uint32_t((p * C + k) * kSlice);
+      copy_async(tv + at * uint32_t(sizeof(TV)), there ? vp + j * kSlice : A.val, there);
+      copy_async(tx + at * uint32_t(sizeof(TX)), there ? x + c[i] : x, there);
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
   };
-  issue(0, 0);
-  issue(1, C);
+  int c[N], cn[N];
+  columns(0, c);
+  columns(C, cn);
+  copy(0, 0, c);
+  copy(1, C, cn);
   TA acc = NEG && ok && q == 0 ? static_cast<TA>(b[row]) : TA(0);
   for (int j0 = 0, p = 0; j0 < w; j0 += C, p ^= 1) {
+    if (j0 + 2 * C < w)
+      columns(j0 + 2 * C, c);
     // this thread's part of the stage has come, then every thread's
     asm volatile("cp.async.wait_group 1;" ::: "memory");
     __syncthreads();
-    if (q == 0 && ok) {
-      const int cnt = min(C, w - j0);
-#pragma unroll 8
-      for (int k = 0; k < cnt; ++k) {
+    if (q == 0) {
+#pragma unroll
+      for (int k = 0; k < C; ++k) { // past the row's end: zeros
         const TA av = static_cast<TA>(sv[p][k][lane]), xv = static_cast<TA>(sx[p][k][lane]);
         acc = NEG ? fma(-av, xv, acc) : fma(av, xv, acc);
       }
     }
     if (j0 + 2 * C < w)
       __syncthreads(); // the stage has been read
-    issue(p, j0 + 2 * C);
+    if (j0 + 2 * C < w)
+      copy(p, j0 + 2 * C, c);
+    else
+      asm volatile("cp.async.commit_group;" ::: "memory");
   }
   if (q != 0 || !ok)
     return;
@@ -2048,9 +2072,7 @@ cluster_barrier()
 // FP64; 8 CTAs 6 to 8 us more. (Counting every value on the receiver's mbarrier
 // in place of the barrier: 27, 37 and 25 us, but nothing then tells a CTA that is
 // ahead that another CTA's threads have read their partial sums, and a wait that
-// ran out would leave values under way.) Solves with a launch per sweep and with
-// this: 80^3 Q2 cells 41.8 and 41.6 ms, 40^3 Q2 cells with a refined ball 43.5
-// and 43.1 ms. Where it is taken: exact_rows.
+// ran out would leave values under way.) Where it is taken: exact_rows.
 // Why nothing is overwritten while it is read: a sweep's last reads of `part`
 // and of the old copy of x come before its cluster barrier, for every thread of
 // every CTA, and the next sweep, which is the next to write `part` and the old
@@ -2079,15 +2101,16 @@ constexpr size_t kExactBytes = 220 * 1024; // shared memory per CTA
 //   27 (Q1, 3D):        1,331 -6.5 -7.5; 2,197 -2.3 -4.2; 3,375 -0.7 (another
 //                       right-hand side: +1.2) -3.5; 4,913 +8.8 +3.5
 //   125 (Q2, 3D):       1,331 -5.2 -4.6; 2,197 +12 +5.2
+// The rows of quadratic elements keep their launches, also where the cluster is a
+// few us faster: their solves take hundreds of steps, which carry the other order
+// of an FP32 row's sum into the solution (up to 1e-4 where 600 steps do not
+// converge); the few steps of a Q1 solve leave 4e-13.
 template<class T>
 constexpr int
 exact_rows(int longest_row)
 {
   const bool fp64 = sizeof(T) == 8;
-  return longest_row <= 16   ? 2048
-         : longest_row <= 26 ? (fp64 ? 0 : 1500)
-         : longest_row <= 32 ? (fp64 ? 2700 : 3700)
-                             : 1500;
+  return longest_row <= 16 ? 2048 : longest_row == 27 ? (fp64 ? 2700 : 3700) : 0;
 }
 
 // x twice, the partial sums, the entries' values and columns

@@ -1,6 +1,7 @@
 """Which coarsest levels' sweeps run in one cluster, told by the launches of a cycle:
 fewer than with a launch per sweep (GB_EXACT_CTAS=0) below the rule's line for a row
-length and precision, the same above it.
+length and precision, the same above it and on the long rows of quadratic elements
+(there the same kernels run: the same bits).
 
 The results differ by the order of a row's sum: at most 125 terms, ten damped sweeps
 and the transfers, 125 * 10 roundings of the result's largest value."""
@@ -49,8 +50,8 @@ def _q1(dim, coarse):
     ("q1_3d_2197", lambda: _q1(3, 6), (True, True)),
     ("q1_3d_3375", lambda: _q1(3, 7), (False, True)),
     ("q1_3d_4913", lambda: _q1(3, 8), (False, False)),
-    ("q2_2d_1225", lambda: structured_q2(2, 17, 2), (False, True)),
-    ("q2_3d_1331", lambda: structured_q2(3, 5, 2), (True, True)),
+    ("q2_2d_1225", lambda: structured_q2(2, 17, 2), (False, False)),
+    ("q2_3d_1331", lambda: structured_q2(3, 5, 2), (False, False)),
     ("q2_3d_2197", lambda: structured_q2(3, 6, 2), (False, False)),
 ])
 def test_rule(name, prob, in_cluster):
@@ -59,6 +60,6 @@ def test_rule(name, prob, in_cluster):
         fewer, a = _cycle(P, None, precision)
         each, b = _cycle(P, "0", precision)
         assert (fewer < each - 5) == expected
-        assert expected or fewer == each
+        assert expected or (fewer == each and np.array_equal(a, b))
         unit = 6e-8 if precision == GB_FP32 else 1.1e-16
         assert np.abs(a - b).max() <= 1250 * unit * np.abs(b).max()
