@@ -25,7 +25,7 @@ namespace gb {
 // warps per SM). Without convection the points are unrolled, so that the
 // reference gradients are constants, the products go through the point's metric
 // w |J| kappa J^-1 J^-T, and the upper half alone is summed: 255 registers with
-// spills -> 228 without, 143 -> 110 us for the hierarchy of 64^3 cells.
+// spills -> 228 without, 143 -> 105 us for the hierarchy of 64^3 cells.
 template<int DIM, bool CONV>
 __global__ void __launch_bounds__(128)
 k_q1_element(int ncells, const int* __restrict__ cells, const double* __restrict__ coords,

@@ -658,7 +658,7 @@ fgmres_graph(Context& c, double* x, const double* b, int prec, gb_solve_info* in
 // reference repeats the pass only for a vector of norm 0, which stays 0.) A step
 // of a 129^2 Q1 problem (18 steps) was 35 launches in 158 us, half of it
 // Gram-Schmidt and the host's read of the flags; it is 26 in 80 us (the solve
-// 2.80 -> 1.54 ms; 57^3 Q1, 12 steps: 2.58 -> 1.88).
+// 2.64 -> 1.48 ms; 57^3 Q1, 12 steps: 2.37 -> 1.87).
 void
 left_setup(Context& c, cudaGraphConditionalHandle hLoop, int use_cond)
 {

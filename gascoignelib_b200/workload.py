@@ -34,7 +34,10 @@ def main(argv=None):
                          "timed alone with the L2 flushed before each (gb_bench_sweep)")
     ap.add_argument("--precision", default="fp64", choices=["fp64", "fp32"])
     ap.add_argument("--problem", default="diffusion", choices=["diffusion", "stokes", "q2", "q2ball"],
-                    help="stokes: 2D Q1/Q1 Stokes with Vanka on (2*2^(refine-1))^2 cells")
+                    help="stokes: Q1/Q1 Stokes with Vanka on 4 * 2^(refine-1) cells per dimension")
+    ap.add_argument("--dim", type=int, default=2, choices=[2, 3], help="of the Stokes problem")
+    ap.add_argument("--coarse", type=int, default=1,
+                    help="coarsest cells per dimension of the diffusion problem")
     ap.add_argument("--smoother", default=None, choices=["jacobi", "vanka", "ilu"],
                     help="override the problem's smoother (ilu: omega 1)")
     ap.add_argument("--assemble", type=int, default=0,
@@ -50,7 +53,7 @@ def main(argv=None):
 
     build_library()
     if a.problem == "stokes":
-        P = structured_stokes(2, 2, a.refine)
+        P = structured_stokes(a.dim, 2, a.refine)
         keys = dict(gmressize=31, omega=1.0)
     elif a.problem in ("q2", "q2ball"):
         from gascoignelib_b200.problem import structured_q2, structured_q2_ball
@@ -58,8 +61,8 @@ def main(argv=None):
              else structured_q2_ball(5, a.refine - 2))
         keys = dict(gmressize=31, omega=0.3, maxiter=600)
     else:
-        kappa, rhs = seeded_inputs(3, 1, a.refine)
-        P = structured_problem(3, 1, a.refine, kappa, rhs)
+        kappa, rhs = seeded_inputs(3, a.coarse, a.refine)
+        P = structured_problem(3, a.coarse, a.refine, kappa, rhs)
         keys = dict(gmressize=21, omega=0.8)
     with Context(0) as ctx:
         ctx.load_problem(P)
